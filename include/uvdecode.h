@@ -446,6 +446,34 @@ int uv_sched_admit(const uv_sched_args* args, const uv_sched_admit_args* pass, v
 int uv_sched_commit(const uv_sched_args* args, void* stream);
 int uv_sched_enqueue(const uv_sched_args* args, int n, void* stream);
 
+/* ---------------------------------------------------------------------------------------------------------------
+ * Fused inference weights from the trainer's parameters (Attention.fuse / MLP.fuse, ultraviolet/model.py:289-300,
+ * :384-386), every matrix of every layer in one launch: d_wqkv = [wq; wk; wv] * qkv_scale, d_gu = [w_gate; w_up],
+ * d_wo = wo * o_scale, d_down = w_down, gates, d_lambdas = the four residual lambdas rounded to dst_dtype, d_xsa =
+ * tanh(xsa_alpha).  fold: the residual lambdas are folded into wo and w_down (the stream of the folded step is x / s, s
+ * the product of the resid_* lambdas so far: d_wo = wo * o_scale * (post_attn / s), likewise d_down).  Bit 0 of *status is
+ * set when a lambda is too small or s leaves the range that stream keeps in dst_dtype.  Parameters are contiguous, all
+ * of src_dtype; at most 32 layers.
+ */
+typedef struct {
+  const void *wq, *wk, *wv, *wo, *w_gate, *w_up, *w_down;
+  const void *ve_gate, *attn_gate, *xsa_alpha;           /* or NULL */
+  const void *qkv_scale, *o_scale, *resid_attn, *post_attn, *resid_mlp, *post_mlp;   /* scalars */
+  void *d_wqkv, *d_wo, *d_gu, *d_down, *d_ve_gate, *d_attn_gate;
+  float *d_lambdas, *d_xsa;
+} uv_fuse_layer;
+
+typedef struct {
+  int src_dtype, dst_dtype, n_layers, d, H, K, hd, f, ve_ch, gate_ch, fold, reserved_;
+  int64_t vocab;
+  const void *embed, *value_embed;
+  void *d_embed, *d_value_embed;
+  int* status;
+  const uv_fuse_layer* h_layers;       /* host array of n_layers entries, copied into the launch */
+} uv_fuse_args;
+
+int uv_fuse_weights(const uv_fuse_args* a, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,56 @@
+"""uv_fuse_weights (the one-launch load_from) against the tensor operations it replaces: same bits, for every pair of
+parameter and engine dtypes, on matrices smaller than a block, not a multiple of it, and whose rows break 16-byte
+alignment, and for a folded and a literal residual stream."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _model(over, dtype, seed=0):
+    from ultraviolet_b200.model import MathLM, make_config
+    torch.manual_seed(seed)
+    m = MathLM(make_config("tiny", xsa=True, **over)).cuda()
+    with torch.no_grad():
+        for p in m.parameters():
+            p.copy_(torch.randn_like(p) * 0.2 if p.dim() else 1.0 + 0.2 * torch.randn_like(p))
+    return m.to(dtype)
+
+
+@pytest.mark.parametrize("over", [{}, dict(d_model=72, d_ff=136, head_dim=64, n_kv_heads=1),
+                                  dict(d_model=200, d_ff=328, vocab_size=1000, n_layers=3, attn_gate_channels=13)])
+@pytest.mark.parametrize("src", [torch.float32, torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("dst", [torch.float16, torch.bfloat16])
+def test_one_launch_gives_the_bits_of_the_tensor_ops(over, src, dst):
+    from ultraviolet_b200.engine import DecodeEngine
+    m = _model(over, src)
+    eng = DecodeEngine.from_model(m, dst)
+    n32 = eng.cfg.n_layers * eng.n32_layer
+    for fold in (True, False):
+        eng.fold = fold
+        with torch.no_grad():
+            eng._fuse_by_tensor_ops(m)
+        want, want32 = eng.arena.clone(), eng.arena32.clone()
+        eng.arena.fill_(7)
+        eng.arena32[:n32].fill_(7)
+        eng.load_from(m)
+        assert eng._fuse_plan["args"] is not None
+        for name, (off, shp) in eng.layout.items():
+            n = torch.Size(shp).numel()
+            assert torch.equal(eng.arena[off:off + n], want[off:off + n]), (name, fold)
+        assert torch.equal(eng.arena32, want32)
+
+
+def test_parameters_it_cannot_take_and_lambdas_it_cannot_fold():
+    from ultraviolet_b200.engine import DecodeEngine
+    m = _model({}, torch.float32)
+    eng = DecodeEngine.from_model(m, torch.bfloat16)
+    want = eng.arena.clone()
+    m.blocks[1].attn.wo.data = m.blocks[1].attn.wo.data.t().contiguous().t()      # not contiguous: tensor operations
+    eng.arena.zero_()
+    eng.load_from(m)
+    assert eng._fuse_plan["args"] is None and torch.equal(eng.arena, want)
+    m.blocks[1].attn.wo.data = m.blocks[1].attn.wo.data.contiguous()
+    m.blocks[2].resid_mlp.data.fill_(1e-3)
+    with pytest.raises(ValueError, match="layer 2"):
+        eng.load_from(m)

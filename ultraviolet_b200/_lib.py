@@ -66,6 +66,22 @@ class PrefillAttnArgs(C.Structure):
     ]
 
 
+class FuseLayer(C.Structure):
+    """uv_fuse_layer (include/uvdecode.h)."""
+    _fields_ = [(n, C.c_void_p) for n in (
+        "wq", "wk", "wv", "wo", "w_gate", "w_up", "w_down", "ve_gate", "attn_gate", "xsa_alpha", "qkv_scale", "o_scale",
+        "resid_attn", "post_attn", "resid_mlp", "post_mlp", "d_wqkv", "d_wo", "d_gu", "d_down", "d_ve_gate",
+        "d_attn_gate", "d_lambdas", "d_xsa")]
+
+
+class FuseArgs(C.Structure):
+    """uv_fuse_args (include/uvdecode.h)."""
+    _fields_ = [(n, C.c_int) for n in ("src_dtype", "dst_dtype", "n_layers", "d", "H", "K", "hd", "f", "ve_ch",
+                                       "gate_ch", "fold", "reserved_")] + [("vocab", C.c_int64)] + \
+               [(n, C.c_void_p) for n in ("embed", "value_embed", "d_embed", "d_value_embed", "status")] + \
+               [("h_layers", C.POINTER(FuseLayer))]
+
+
 class SchedArgs(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in (
         "req", "fed", "gen", "cur_tok", "pos", "starts", "row_key", "step_ctr", "samp_tok", "samp_lp", "prompt_off",
@@ -133,6 +149,7 @@ SIGNATURES = {
                                  C.c_void_p]),
     "uv_gemm_resid_norm": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p,
                                      C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]),
+    "uv_fuse_weights": (C.c_int, [C.POINTER(FuseArgs), C.c_void_p]),
     "uv_sched_step": (C.c_int, [C.POINTER(SchedArgs), C.c_void_p]),
     "uv_sched_admit": (C.c_int, [C.POINTER(SchedArgs), C.POINTER(SchedAdmitArgs), C.c_void_p]),
     "uv_sched_enqueue": (C.c_int, [C.POINTER(SchedArgs), C.c_int, C.c_void_p]),

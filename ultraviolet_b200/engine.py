@@ -17,6 +17,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import weakref
 
 import torch
 from torch import Tensor
@@ -72,6 +73,8 @@ class DecodeEngine:
         if cfg.rope_pairs:
             self.inv_freq.copy_((1.0 / cfg.rope_base) ** torch.linspace(0, 1, cfg.rope_pairs, dtype=torch.float32))
         self._scratch: dict[int, dict] = {}
+        self._fuse_plan = None      # load_from's launch arguments for the parameter tensors it saw last
+        self._fuse_status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.version = 0
         # GEMMs with fused epilogues (csrc/gemm_fused.cu).  Correct, but measured SLOWER than cuBLAS + the separate row
         # kernels on B200 at decode batch sizes (per pair 8-20 us against 6-8 us: four warps of straight-line code per
@@ -128,7 +131,73 @@ class DecodeEngine:
     @torch.no_grad()
     def load_from(self, model) -> None:
         """(Re)compute every fused weight from the model's parameters INTO the existing arena (same formulas and
-        rounding as Attention.fuse / MLP.fuse; pointers never change)."""
+        rounding as Attention.fuse / MLP.fuse; pointers never change).  One launch (uv_fuse_weights) where the
+        parameters are contiguous tensors of one dtype on this device, tensor operations otherwise."""
+        if not self._fuse_launch(model):
+            self._fuse_by_tensor_ops(model)
+        self.version += 1
+
+    def _fuse_launch(self, model) -> bool:
+        """load_from as one kernel launch; False when it does not apply or when a residual lambda cannot be folded
+        (_fuse_by_tensor_ops then says which)."""
+        mods = [m for b in model.blocks for m in (b, b.attn, b.mlp)]
+        params = [model.embed.weight, model.value_embed.weight if self.use_ve else None]
+        params += [q for m in mods for q in m._parameters.values()]
+        params = [q for q in params if q is not None]
+        ptrs = [q.data_ptr() for q in params]
+        plan = self._fuse_plan
+        if (plan is None or plan["ptrs"] != ptrs or plan["fold"] != self.fold
+                or any(r() is not q for r, q in zip(plan["refs"], params))):
+            plan = self._fuse_plan = self._plan_fuse(model, ptrs, [weakref.ref(q) for q in params])
+        if plan["args"] is None:
+            return False
+        with torch.cuda.device(self.device):
+            self._fuse_status.zero_()
+            _lib.check(_lib.lib().uv_fuse_weights(C.byref(plan["args"]), stream_ptr(self.device)), "uv_fuse_weights")
+        return not self.fold or int(self._fuse_status.item()) == 0
+
+    def _plan_fuse(self, model, ptrs, refs) -> dict:
+        """Arguments of uv_fuse_weights for these parameter tensors (kept as long as the same tensors come back:
+        walking a few hundred attributes costs more than the kernel)."""
+        cfg, w = self.cfg, self.w
+        plan = dict(ptrs=ptrs, refs=refs, fold=self.fold, args=None)
+        dt = model.embed.weight.dtype
+        ok = dt in (torch.float32, torch.float16, torch.bfloat16) and cfg.n_layers <= 32
+
+        def src(t):
+            nonlocal ok
+            ok = ok and torch.is_tensor(t) and t.dtype == dt and t.device == self.arena.device and t.is_contiguous()
+            return t.data_ptr() if ok else None
+        layers = (_lib.FuseLayer * cfg.n_layers)()
+        for l, (blk, y) in enumerate(zip(model.blocks, layers)):
+            at, mlp = blk.attn, blk.mlp
+            y.wq, y.wk, y.wv, y.wo = src(at.wq), src(at.wk), src(at.wv), src(at.wo)
+            y.w_gate, y.w_up, y.w_down = src(mlp.w_gate), src(mlp.w_up), src(mlp.w_down)
+            y.qkv_scale, y.o_scale = src(at.qkv_scale), src(at.o_scale)
+            y.resid_attn, y.post_attn = src(blk.resid_attn), src(blk.post_attn)
+            y.resid_mlp, y.post_mlp = src(blk.resid_mlp), src(blk.post_mlp)
+            y.d_wqkv, y.d_wo, y.d_gu, y.d_down = (w[f"l{l}.{n}"].data_ptr() for n in ("wqkv", "wo", "gu", "down"))
+            y.d_lambdas = self.lambdas[l].data_ptr()
+            if cfg.has_ve(l):
+                y.ve_gate, y.d_ve_gate = src(at.ve_gate), w[f"l{l}.ve_gate"].data_ptr()
+            if cfg.gate_channels:
+                y.attn_gate, y.d_attn_gate = src(at.attn_gate), w[f"l{l}.attn_gate"].data_ptr()
+            if cfg.xsa:
+                y.xsa_alpha, y.d_xsa = src(at.xsa_alpha), self.xsa[l].data_ptr()
+        a = _lib.FuseArgs()
+        a.embed, a.d_embed = src(model.embed.weight), w["embed"].data_ptr()
+        if self.use_ve:
+            a.value_embed, a.d_value_embed = src(model.value_embed.weight), w["value_embed"].data_ptr()
+        if not ok or len(model.blocks) != cfg.n_layers:
+            return plan
+        a.src_dtype, a.dst_dtype, a.n_layers, a.fold = DTYPE_CODE[dt], DTYPE_CODE[self.dtype], cfg.n_layers, int(self.fold)
+        a.d, a.H, a.K, a.hd, a.f = cfg.d_model, cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, cfg.d_ff
+        a.ve_ch, a.gate_ch, a.vocab = cfg.ve_gate_channels, cfg.gate_channels, cfg.vocab_size
+        a.status, a.h_layers = self._fuse_status.data_ptr(), layers
+        plan["args"] = a
+        return plan
+
+    def _fuse_by_tensor_ops(self, model) -> None:
         cfg, dt, w = self.cfg, self.dtype, self.w
         w["embed"].copy_(model.embed.weight)
         if self.use_ve:
@@ -163,7 +232,6 @@ class DecodeEngine:
             self.lambdas[l].copy_(lam.to(dt).float())  # Block.finish casts each scalar to the activation dtype
             if cfg.xsa:
                 self.xsa[l].copy_(torch.tanh(at.xsa_alpha.detach().float()))
-        self.version += 1
 
     def nbytes(self) -> int:
         return self.arena.numel() * self.arena.element_size() + self.arena32.numel() * 4
