@@ -1,0 +1,88 @@
+"""The row kernels that launches of many rows take (a warp a row) against the ones that launches of few rows take, on the
+same rows handed over in one call and in pieces: around the row count where the choice changes, on the last rows of a
+block, on every head width, with and without gates, value embedding, rotation and cache append."""
+import ctypes as C
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _pieces(n, cut):
+    return [(a, min(a + cut, n)) for a in range(0, n, cut)]
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,d,f", [(768, 640, 1664), (769, 64, 128), (1003, 1032, 4096)])
+def test_swiglu_of_many_rows(dtype, n, d, f):
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.kernels._util import DTYPE_CODE, stream_ptr
+    g = torch.Generator(device="cuda").manual_seed(n)
+    gu = torch.randn(n, 2 * f, device="cuda", generator=g).to(dtype)
+    h = (torch.randn(n, d, device="cuda", generator=g) * 3).to(dtype)
+    got, want = (torch.zeros(n, f, device="cuda", dtype=dtype) for _ in range(2))
+    for out, cut in ((got, n), (want, 256)):
+        for a, b in _pieces(n, cut):
+            _lib.check(_lib.lib().uv_swiglu_rs(gu[a:b].data_ptr(), h[a:b].data_ptr(), DTYPE_CODE[dtype], d, f,
+                                               out[a:b].data_ptr(), b - a, stream_ptr(gu.device)), "uv_swiglu_rs")
+    rs = torch.rsqrt(h.float().pow(2).mean(1, keepdim=True) + 2.0 ** -23)
+    x = gu.float() * rs
+    ref = torch.nn.functional.silu(x[:, :f]) * x[:, f:]
+    tol = 2e-2 if dtype == torch.bfloat16 else 3e-3
+    assert torch.allclose(got.float(), ref, rtol=tol, atol=tol * ref.abs().max().item() * 1e-2)
+    assert (got != want).float().mean() < 1e-3       # (norm factors summed in another order: rare last-bit differences)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,H,K,hd,d,pairs,gate,ve,ring", [
+    (768, 8, 1, 64, 640, 16, 128, 12, True), (1001, 8, 1, 64, 640, 0, 128, 0, False), (770, 4, 2, 64, 64, 16, 16, 4, True),
+    (800, 3, 1, 128, 1040, 32, 0, 5, False), (900, 6, 2, 32, 192, 8, 24, 12, True)])
+def test_qkv_post_of_many_rows(dtype, n, H, K, hd, d, pairs, gate, ve, ring):
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.kernels._util import DTYPE_CODE, stream_ptr
+    g = torch.Generator(device="cuda").manual_seed(n)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    S, rows, vocab = 40, 64, 50
+    x, qkv0 = (rnd(n, d) * 2).to(dtype), rnd(n, (H + 2 * K) * hd).to(dtype)
+    tok = torch.randint(-2, vocab + 2, (n,), device="cuda", generator=g)
+    perm = torch.randperm(rows * (30 if ring else S), device="cuda", generator=g)[:n]     # no two entries share a slot
+    row, pos = perm % rows, perm // rows
+    pos = pos + (S * 3 if ring else 0)
+    if not ring:
+        pos[5] = S + 2                                                                    # past the cache: counted
+    last = torch.where(torch.rand(n, device="cuda", generator=g) < 0.1, pos + S, pos)     # overwritten within the launch
+    gw, vw, emb = rnd(H, max(gate, 1)).to(dtype), rnd(K, max(ve, 1)).to(dtype), rnd(vocab, K * hd).to(dtype)
+    inv = torch.rand(max(pairs, 1), device="cuda", generator=g)
+    cs = torch.cat([torch.cos(pos[:, None] * inv), torch.sin(pos[:, None] * inv)], 1).to(dtype).float().contiguous()
+    res = []
+    for cut in (n, 250):
+        qkv = qkv0.clone()
+        gates = torch.zeros(n, H, device="cuda")
+        kc, vc = (torch.zeros(rows, K, S, hd, dtype=torch.int8, device="cuda") for _ in range(2))
+        ks, vs = (torch.zeros(rows, K, S, dtype=torch.float16, device="cuda") for _ in range(2))
+        oob = torch.zeros(1, dtype=torch.int32, device="cuda")
+        for a, b in _pieces(n, cut):
+            q = _lib.QkvArgs()
+            q.qkv, q.xn, q.tok, q.pos = (t[a:b].data_ptr() for t in (qkv, x, tok, pos))
+            q.row_map, q.last_pos = row[a:b].data_ptr(), last[a:b].data_ptr()
+            q.k_cache, q.v_cache, q.k_scale, q.v_scale = kc.data_ptr(), vc.data_ptr(), ks.data_ptr(), vs.data_ptr()
+            q.oob_count, q.dtype, q.vocab, q.xn_raw, q.ring = oob.data_ptr(), DTYPE_CODE[dtype], vocab, 1, int(ring)
+            q.B, q.H, q.K, q.hd, q.d, q.S, q.S_alloc, q.n_pairs = b - a, H, K, hd, d, S, S, pairs
+            if pairs:
+                q.inv_freq, q.rope_cs = inv.data_ptr(), cs[a:b].data_ptr()
+            if ve:
+                q.ve_gate, q.value_embed, q.ve_ch = vw.data_ptr(), emb.data_ptr(), ve
+            if gate:
+                q.gate_w, q.gate_out, q.gate_ch = gw.data_ptr(), gates[a:b].data_ptr(), gate
+            _lib.check(_lib.lib().uv_qkv_post_args(C.byref(q), stream_ptr(x.device)), "uv_qkv_post")
+        res.append((qkv, gates, kc, vc, ks, vs, oob))
+    (q1, g1, *c1, o1), (q2, g2, *c2, o2) = res
+    assert int(o1) == int(o2) == (0 if ring else 2 * K)
+    ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
+    assert torch.allclose(q1.float(), q2.float(), rtol=2 * ulp, atol=2 * ulp) and (q1 != q2).float().mean() < 5e-3
+    assert torch.allclose(g1, g2, rtol=2 * ulp, atol=2 * ulp)
+    for a, b in zip(c1[:2], c2[:2]):
+        assert (a.int() - b.int()).abs().max() <= 1 and (a != b).float().mean() < 1e-2
+    for a, b in zip(c1[2:], c2[2:]):
+        assert torch.equal(a == 0, b == 0) and torch.allclose(a.float(), b.float(), rtol=2 * ulp, atol=0)

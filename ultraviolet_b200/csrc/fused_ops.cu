@@ -28,6 +28,17 @@ template <typename T> __device__ __forceinline__ void st2(T* p, float a, float b
   *reinterpret_cast<typename Vec2<T>::type*>(p) = v;
 }
 
+// two values at a time through the packed converters (the scalar ones go to a quarter-rate unit)
+template <typename T> __device__ __forceinline__ typename Vec2<T>::type pair(float a, float b);
+template <> __device__ __forceinline__ __half2 pair<__half>(float a, float b) { return __floats2half2_rn(a, b); }
+template <> __device__ __forceinline__ __nv_bfloat162 pair<__nv_bfloat16>(float a, float b) {
+  return __floats2bfloat162_rn(a, b);
+}
+template <typename T> __device__ __forceinline__ float2 rnd2(float a, float b) {
+  const typename Vec2<T>::type v = pair<T>(a, b);
+  return make_float2(to_f32<T>(v.x), to_f32<T>(v.y));
+}
+
 // ------------------------------------------------------------------------------------------------ embed + norms
 // A warp owns a row; rows of up to ROW_MAX elements live in registers as 16-byte vectors (lane owns elements
 // 8*lane + 256*j .. +7): one global read and one write per element, three or four memory instructions per lane.
@@ -253,6 +264,58 @@ __global__ void __launch_bounds__(SWR_THREADS) swiglu_rs_kernel(const T* __restr
   }
 }
 
+// The same for launches of many rows: a warp owns a row, requests all of it (16-byte pieces of h, g and u) before it
+// uses any, and forms rs once.  At prefill sizes the kernel above is bound by its own traffic -- four CTAs a row read
+// h four times and leave 48 bytes a thread in flight; this one streams.  20,500 rows of f = 1664: 99 us -> 43 us
+// (230 MB: 35 us at the measured copy rate).
+constexpr int SWM_WARPS = 8;
+constexpr int SWM_ROWS = 768;
+constexpr int SWM_V = 7;      // 8-feature vectors a lane holds at a time
+
+template <typename T>
+__global__ void __launch_bounds__(SWM_WARPS * 32) swiglu_rows_kernel(const T* __restrict__ gu, const T* __restrict__ hrow,
+                                                                     int d, int f, T* __restrict__ act, int B) {
+  const int lane = threadIdx.x & 31, row = blockIdx.x * SWM_WARPS + (threadIdx.x >> 5);
+  pdl_wait();
+  pdl_trigger();
+  if (row >= B) return;
+  const T* g = gu + (int64_t)row * 2 * f;
+  const int nvec = f / 8;
+  uint4 gv[SWM_V], uv[SWM_V];
+  auto request = [&](int v0) {
+#pragma unroll
+    for (int j = 0; j < SWM_V; ++j) {
+      const int v = v0 + 32 * j + lane;
+      if (v < nvec) {
+        gv[j] = __ldcs(reinterpret_cast<const uint4*>(g) + v);
+        uv[j] = __ldcs(reinterpret_cast<const uint4*>(g + f) + v);
+      }
+    }
+  };
+  request(0);
+  const float rs = row_rms_factor<T>(hrow + (int64_t)row * d, d, lane);
+  for (int v0 = 0; v0 < nvec; v0 += 32 * SWM_V) {
+    if (v0) request(v0);
+#pragma unroll
+    for (int j = 0; j < SWM_V; ++j) {
+      const int v = v0 + 32 * j + lane;
+      if (v >= nvec) break;
+      const typename Vec2<T>::type *a = reinterpret_cast<const typename Vec2<T>::type*>(&gv[j]),
+                                   *b = reinterpret_cast<const typename Vec2<T>::type*>(&uv[j]);
+      uint4 out;
+      typename Vec2<T>::type* o = reinterpret_cast<typename Vec2<T>::type*>(&out);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float2 g2 = rnd2<T>(to_f32<T>(a[k].x) * rs, to_f32<T>(a[k].y) * rs);
+        const float2 u2 = rnd2<T>(to_f32<T>(b[k].x) * rs, to_f32<T>(b[k].y) * rs);
+        const float2 s = rnd2<T>(__fdividef(g2.x, 1.0f + __expf(-g2.x)), __fdividef(g2.y, 1.0f + __expf(-g2.y)));
+        o[k] = pair<T>(s.x * u2.x, s.y * u2.y);
+      }
+      *(reinterpret_cast<uint4*>(act + (int64_t)row * f) + v) = out;
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------------ QKV post
 // One warp per (row b, head slot), in place on the packed GEMM output; the arithmetic lives in qkv_post.cuh.
 // W warps per CTA, one (row, item) per warp.  COOP (xn_raw launches whose items per row are a multiple of W): the W
@@ -331,10 +394,226 @@ __global__ void __launch_bounds__(W * 32) qkv_post_kernel(const __grid_constant_
   if (appends) qkv_post_append<T, HD>(P, b, hs, lane, x, &dest);
 }
 
+// The same for launches of many rows (xn_raw, RoPE from the table): a warp owns a row -- the norm factor is formed once
+// from registers that then feed the gates -- and a head slot is a group of HD / 8 lanes with 16 bytes each, so a row of
+// ten 64-wide slots is three passes.  The kernel above spends a warp on every slot and gate, eighteen a row, each with
+// its own chain of loads: right when rows are few, three times the instructions and 2-byte-a-lane traffic when they are
+// not.  20,500 rows: 136 us -> 43 us (78 MB: 12 us at the measured copy rate).
+constexpr int QPR_WARPS = 8;
+constexpr int QPR_ROWS = 768;
+constexpr int QPR_GCH = 128;   // channels a gate may read
+
+template <typename T, int HD>
+__global__ void __launch_bounds__(QPR_WARPS * 32) qkv_post_rows_kernel(const __grid_constant__ QkvPostParams P) {
+  constexpr int LG = HD / 8, NG = 32 / LG;              // lanes a slot, slots a pass
+  extern __shared__ __align__(16) unsigned char qpr_smem[];
+  T* const gw = reinterpret_cast<T*>(qpr_smem);         // (H, gate_ch) then (K, ve_ch)
+  T* const vw = gw + (P.gate_out ? P.H * P.gate_ch : 0);
+  const int lane = threadIdx.x & 31, grp = lane / LG, gl = lane % LG;
+  const int slots = P.H + 2 * P.K;
+  if (P.gate_out)
+    for (int i = threadIdx.x; i < P.H * P.gate_ch; i += QPR_WARPS * 32) gw[i] = static_cast<const T*>(P.gate_w)[i];
+  if (P.ve_gate)
+    for (int i = threadIdx.x; i < P.K * P.ve_ch; i += QPR_WARPS * 32) vw[i] = static_cast<const T*>(P.ve_gate)[i];
+  pdl_wait();
+  pdl_trigger();
+  __syncthreads();
+  auto unpack = [](const uint4& u, float (&v)[8]) {
+    const typename Vec2<T>::type* h = reinterpret_cast<const typename Vec2<T>::type*>(&u);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[2 * k] = to_f32<T>(h[k].x), v[2 * k + 1] = to_f32<T>(h[k].y);
+  };
+  auto pack = [](const float (&v)[8]) {
+    uint4 u;
+    typename Vec2<T>::type* h = reinterpret_cast<typename Vec2<T>::type*>(&u);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) h[k] = pair<T>(v[2 * k], v[2 * k + 1]);
+    return u;
+  };
+  auto scale = [](float (&v)[8], float s) {
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+      const float2 r = rnd2<T>(v[k] * s, v[k + 1] * s);
+      v[k] = r.x, v[k + 1] = r.y;
+    }
+  };
+  auto group_sum = [](float v) {
+#pragma unroll
+    for (int o = LG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  };
+  auto group_max = [](float v) {
+#pragma unroll
+    for (int o = LG / 2; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+  };
+  for (int b = blockIdx.x * QPR_WARPS + (threadIdx.x >> 5); b < P.B; b += gridDim.x * QPR_WARPS) {
+    const T* xr = static_cast<const T*>(P.xn) + (int64_t)b * P.d;
+    T* const qr = static_cast<T*>(P.qkv) + (int64_t)b * slots * HD;
+    uint4 xu[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int i = 8 * lane + 256 * j;
+      xu[j] = i < P.d ? *reinterpret_cast<const uint4*>(xr + i) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    uint4 raw = grp < slots ? *reinterpret_cast<const uint4*>(qr + grp * HD + 8 * gl) : make_uint4(0u, 0u, 0u, 0u);
+    const QkvSlot dest = qkv_post_slot(P, b);
+    const float* cs = P.inv_freq ? P.rope_cs + (int64_t)b * 2 * P.n_pairs : nullptr;
+    float ss = 0.f, x[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      unpack(xu[j], x);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) ss += x[k] * x[k];
+    }
+    for (int i = 8 * lane + 1024; i < P.d; i += 256) {  // rows wider than 1024 elements
+      unpack(*reinterpret_cast<const uint4*>(xr + i), x);
+#pragma unroll
+      for (int k = 0; k < 8; ++k) ss += x[k] * x[k];
+    }
+    const float rs = rsqrtf(warp_sum(ss) / (float)P.d + RMS_EPS);
+    // ---- gates: the row's first 128 channels, normalised, 8 in each lane of both half-warps
+    float xc[8];
+    {
+      const uint4 u = make_uint4(__shfl_sync(0xffffffffu, xu[0].x, lane & 15), __shfl_sync(0xffffffffu, xu[0].y, lane & 15),
+                                 __shfl_sync(0xffffffffu, xu[0].z, lane & 15), __shfl_sync(0xffffffffu, xu[0].w, lane & 15));
+      unpack(u, xc);
+      scale(xc, rs);
+    }
+    if (P.gate_out) {
+      const int c = 8 * (lane & 15);
+      for (int h0 = 0; h0 < P.H; h0 += 2) {             // a head per half-warp
+        const int h = h0 + (lane >> 4);
+        float acc = 0.f;
+        if (h < P.H && c < P.gate_ch) {
+          float w[8];
+          unpack(*reinterpret_cast<const uint4*>(gw + h * P.gate_ch + c), w);
+#pragma unroll
+          for (int k = 0; k < 8; ++k) acc += xc[k] * w[k];
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        acc = rnd<T>(acc);
+        const float g = rnd<T>(2.0f * rnd<T>(__fdividef(1.0f, 1.0f + __expf(-acc))));
+        if (h < P.H && (lane & 15) == 0) P.gate_out[(int64_t)b * P.H + h] = g;
+      }
+    }
+    // ---- head slots, NG at a time
+    for (int s0 = 0; s0 < slots; s0 += NG) {
+      const int hs = s0 + grp;
+      const bool live = hs < slots, isv = hs >= P.H + P.K;
+      const uint4 cur = raw;
+      if (s0 + NG < slots)
+        raw = hs + NG < slots ? *reinterpret_cast<const uint4*>(qr + (hs + NG) * HD + 8 * gl) : make_uint4(0u, 0u, 0u, 0u);
+      unpack(cur, x);
+      scale(x, rs);
+      ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) ss += x[k] * x[k];
+      const float inv = rsqrtf(group_sum(ss) / (float)HD + RMS_EPS);
+      if (!isv) scale(x, inv);
+      if (cs != nullptr) {                              // dim j < n_pairs turns with dim j + n_pairs
+        const int np8 = P.n_pairs / 8;
+        const bool turns = !isv && gl < 2 * np8;
+        const float* c = cs + 8 * (gl & (np8 - 1));
+        const float sgn = gl < np8 ? -1.f : 1.f;        // x1 c - x2 s, x1 s + x2 c: every product and sum rounded
+#pragma unroll
+        for (int k = 0; k < 8; k += 2) {
+          const float o0 = __shfl_xor_sync(0xffffffffu, x[k], np8), o1 = __shfl_xor_sync(0xffffffffu, x[k + 1], np8);
+          if (turns) {
+            const float2 cc = *reinterpret_cast<const float2*>(c + k), sn = *reinterpret_cast<const float2*>(c + P.n_pairs + k);
+            const float2 a = rnd2<T>(x[k] * cc.x, x[k + 1] * cc.y), d = rnd2<T>(o0 * sn.x, o1 * sn.y);
+            const float2 y = rnd2<T>(a.x + sgn * d.x, a.y + sgn * d.y);
+            x[k] = y.x, x[k + 1] = y.y;
+          }
+        }
+      }
+      if (P.ve_gate != nullptr && s0 + NG > P.H + P.K) {  // some slot of this pass is a value head (warp-uniform)
+        const int kh = isv && live ? hs - P.H - P.K : 0;
+        float acc = 0.f;                                // channels 8 i .. 8 i + 7 sit in lane i
+        for (int k0 = 0; k0 < P.K; ++k0) {
+          float p = 0.f;
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (lane < 16 && 8 * lane + k < P.ve_ch) p += xc[k] * to_f32<T>(vw[k0 * P.ve_ch + 8 * lane + k]);
+          p = warp_sum(p);
+          if (k0 == kh) acc = p;
+        }
+        if (isv && live) {
+          acc = rnd<T>(acc);
+          const float g = rnd<T>(2.0f * rnd<T>(__fdividef(1.0f, 1.0f + __expf(-acc))));
+          int64_t t = P.tok[b];
+          if (t < 0 || t >= P.vocab) t = 0;
+          float ve[8];
+          unpack(*reinterpret_cast<const uint4*>(static_cast<const T*>(P.value_embed) + (t * P.K + kh) * HD + 8 * gl), ve);
+#pragma unroll
+          for (int k = 0; k < 8; k += 2) {
+            const float2 a = rnd2<T>(g * ve[k], g * ve[k + 1]), y = rnd2<T>(x[k] + a.x, x[k + 1] + a.y);
+            x[k] = y.x, x[k + 1] = y.y;
+          }
+        }
+      }
+      if (live) *reinterpret_cast<uint4*>(qr + hs * HD + 8 * gl) = pack(x);
+      if (P.k_cache != nullptr && s0 + NG > P.H) {      // quantise + append (quantize_lane, common.cuh, 8 values a lane)
+        float amax = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(x[k]));
+        amax = group_max(amax);
+        if (live && hs >= P.H) {
+          int64_t p = dest.pos;
+          bool keep = true;
+          if (P.ring) {
+            keep = !(dest.last >= 0 && p + P.S <= dest.last);   // else a newer token of this launch owns the slot
+            p = ((p % P.S) + P.S) % P.S;
+          }
+          if (keep && (p < 0 || p >= P.S)) {
+            keep = false;
+            if (gl == 0 && P.oob) atomicAdd(P.oob, 1);
+          }
+          if (keep) {
+            const __half s16 = __float2half_rn(__fdiv_rn(amax, 127.0f));
+            const float sf = fmaxf(__half2float(s16), 1e-30f);
+            uint32_t w8[2] = {0u, 0u};
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+              const float r = fminf(fmaxf(rintf(__fdiv_rn(x[k], sf)), -127.0f), 127.0f);
+              w8[k / 4] |= ((uint32_t)__float2int_rn(r) & 0xffu) << (8 * (k & 3));
+            }
+            const int kh = isv ? hs - P.H - P.K : hs - P.H;
+            const int64_t dst = (dest.row * P.K + kh) * P.S_alloc + p;
+            *reinterpret_cast<uint2*>((isv ? P.v_cache : P.k_cache) + dst * HD + 8 * gl) = make_uint2(w8[0], w8[1]);
+            if (gl == 0) (isv ? P.v_scale : P.k_scale)[dst] = __half_as_ushort(s16);
+          }
+        }
+      }
+    }
+  }
+}
+
 template <typename T>
 static int launch_qkv_post(const QkvPostParams& P, int hd, cudaStream_t st) {
   const int per_row = P.H + 2 * P.K + (P.gate_out ? P.H : 0);
   const int64_t items = (int64_t)P.B * per_row;
+  // many rows: a warp a row.  Below QPR_ROWS rows a row's own chain is what counts, and a warp for every slot shortens it
+  // (256 rows: 4.2 us against 7.0; 768: 7.7 against 7.3; 4096: 12.9 with this one).
+  const bool rows_ok = P.B >= QPR_ROWS && P.xn_raw && (!P.gate_out || (P.gate_ch <= QPR_GCH && P.gate_ch % 8 == 0)) &&
+                       (!P.ve_gate || P.ve_ch <= QPR_GCH) && aligned16(P.qkv) &&
+                       (!P.ve_gate || aligned16(P.value_embed)) &&
+                       (!P.k_cache || (((uintptr_t)P.k_cache | (uintptr_t)P.v_cache) & 7) == 0) &&
+                       (!P.inv_freq || (P.rope_cs && (P.n_pairs == 8 || P.n_pairs == 16 || P.n_pairs == 32 || P.n_pairs == 64)));
+  if (rows_ok) {
+    const size_t smem = ((P.gate_out ? (size_t)P.H * P.gate_ch : 0) + (P.ve_gate ? (size_t)P.K * P.ve_ch : 0)) * sizeof(T);
+    const int64_t ctas = ((int64_t)P.B + QPR_WARPS - 1) / QPR_WARPS;
+    const unsigned grid = (unsigned)(ctas < 148 * 6 ? ctas : 148 * 6);
+    switch (hd) {
+      case 16: launch_pdl(qkv_post_rows_kernel<T, 16>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
+      case 32: launch_pdl(qkv_post_rows_kernel<T, 32>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
+      case 64: launch_pdl(qkv_post_rows_kernel<T, 64>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
+      case 128: launch_pdl(qkv_post_rows_kernel<T, 128>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
+      default: return UV_ERR_SHAPE;
+    }
+    return check_launch();
+  }
   // cooperative row reduction when the launch defers the norm and a row's items fill whole CTAs of 6 or 4 warps
   static const bool coop_on = [] {
     const char* v = getenv("UVDECODE_QKV_POST_COOP");
@@ -472,6 +751,19 @@ extern "C" int uv_swiglu_rs(const void* gu, const void* h, int dtype, int d, int
   if (f < 8 || (f & 7) || f > 8 * SWR_THREADS * SWR_VMAX * SWR_SPLIT || d < 8 || (d & 7)) return UV_ERR_SHAPE;
   if (!aligned16(h) || !aligned16(gu) || !aligned16(act)) return UV_ERR_ALIGN;  // rows move as 16-byte vectors
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  // From SWM_ROWS rows on the launch is bound by what it moves; below, by one row's chain of loads, which four CTAs a row
+  // shorten (256 rows: 3.2 us against 4.9; 768: 5.2 against 5.0; 2048: 6.3 with this one).
+  if (B >= SWM_ROWS) {
+    const dim3 grid((unsigned)((B + SWM_WARPS - 1) / SWM_WARPS)), block(SWM_WARPS * 32);
+    if (dtype == UV_F16)
+      launch_pdl(swiglu_rows_kernel<__half>, grid, block, 0, st, static_cast<const __half*>(gu),
+                 static_cast<const __half*>(h), d, f, static_cast<__half*>(act), B);
+    else if (dtype == UV_BF16)
+      launch_pdl(swiglu_rows_kernel<__nv_bfloat16>, grid, block, 0, st, static_cast<const __nv_bfloat16*>(gu),
+                 static_cast<const __nv_bfloat16*>(h), d, f, static_cast<__nv_bfloat16*>(act), B);
+    else return UV_ERR_DTYPE;
+    return check_launch();
+  }
   if (dtype == UV_F16)
     launch_pdl(swiglu_rs_kernel<__half>, dim3((unsigned)B * SWR_SPLIT), dim3(SWR_THREADS), 0, st, static_cast<const __half*>(gu),
                static_cast<const __half*>(h), d, f, static_cast<__half*>(act));
