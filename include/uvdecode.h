@@ -474,6 +474,20 @@ typedef struct {
 
 int uv_fuse_weights(const uv_fuse_args* a, void* stream);
 
+/* ---------------------------------------------------------------------------------------------------------------
+ * A left-padded prompt batch as one packed pass (the packed route of prefill, ultraviolet/kernels/fast_decode.py:117-163):
+ * prompt i is idx[i, starts[i] .. T - 1] (row stride ld).  Writes the prefix sums cu / tile_cu (n + 1) that uv_prefill_attn
+ * walks and, per packed row, its token, position (that of the padded frame), cache row rows[i] and last position T - 1.
+ * M is the sum of the prompts' lengths.
+ */
+int uv_pack_prompts(const int64_t* idx, int64_t ld, int T, const int64_t* starts, const int64_t* rows, int n, int64_t M,
+                    int32_t* cu, int32_t* tile_cu, int64_t* tok, int64_t* pos, int64_t* row, int64_t* last, void* stream);
+/* out[i] = rms_norm(x[cu[i + 1] - 1]) for each of n packed sequences (zeros for an empty one): the final norm of what the
+ * LM head reads (fast_decode.py:332-334). */
+int uv_gather_norm(const void* x, int dtype, int d, const int32_t* cu, int n, void* out, void* stream);
+/* out = a * sigmoid((x + b) / c), fp32, of the (B, V) raw head output (MathLM.logits, ultraviolet/model.py:824-827). */
+int uv_softcap(const void* x, int dtype, int64_t n, float a, float b, float c, float* out, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

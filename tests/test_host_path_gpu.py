@@ -1,0 +1,80 @@
+"""The native host paths against the Python ones they stand in for: same launches, so the same bits; and the launches
+around a packed prompt pass (offsets, packing, last-token norm, softcap) at the sizes where they can go wrong."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("B,S,window,dtype,splits", [(1, 40, 0, torch.float16, None), (37, 900, 0, torch.bfloat16, None),
+                                                     (5, 256, 256, torch.bfloat16, None), (3, 4096, 0, torch.float16, 12)])
+def test_decode_attention_host_path(B, S, window, dtype, splits):
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.kernels import decode_attention
+    from ultraviolet_b200.kernels.decode_attn import _decode_attn_op, default_splits
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q = torch.randn(B, 8, 64, device="cuda", generator=g).to(dtype)
+    k, v = (torch.randint(-127, 128, (B, 1, S, 64), device="cuda", generator=g, dtype=torch.int8) for _ in range(2))
+    ks, vs = (torch.rand(B, 1, S, device="cuda", generator=g).half() * 0.02 for _ in range(2))
+    pos = torch.randint(0, S, (B,), device="cuda", generator=g)
+    st = torch.zeros(B, dtype=torch.long, device="cuda")
+    args = (q, k, v, pos, st, 0.14)
+    native = _lib.host().decode_attention(*args, window, -1, ks, vs, 0, splits or -2 ** 31)
+    assert native is not None
+    n = splits or default_splits(B, min(S, window) if window else S, q.device)
+    want = _decode_attn_op(*args, window, window > 0, ks, vs, n)
+    assert torch.equal(native, want)
+    assert torch.equal(decode_attention(*args, window=window, k_scale=ks, v_scale=vs, num_splits=splits), want)
+    # what it does not take goes to the op: gradients wanted, other index types, a dispatch mode
+    assert _lib.host().decode_attention(q.clone().requires_grad_(), k, v, pos, st, 0.14, window, -1, ks, vs, 0, 1) is None
+    assert torch.equal(decode_attention(q, k, v, pos.int(), st, 0.14, window=window, k_scale=ks, v_scale=vs,
+                                        num_splits=n), want)
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    with FakeTensorMode() as mode:
+        fake = [mode.from_tensor(t) for t in (q, k, v, pos, st, ks, vs)]
+        out = decode_attention(*fake[:5], 0.14, window=window, k_scale=fake[5], v_scale=fake[6], num_splits=n)
+        assert out.shape == q.shape
+    with pytest.raises(RuntimeError):
+        decode_attention(*args, window=window, k_scale=ks, v_scale=vs, num_splits=-1)
+
+
+@pytest.mark.parametrize("lens,T", [([1], 1), ([0, 5, 16, 17, 0], 17), (list(range(1500)), 1500)])
+def test_prompt_packing(lens, T):
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.fast_decode import pack_prompts
+    from ultraviolet_b200.kernels._util import stream_ptr
+    n, dev = len(lens), "cuda"
+    lens = np.minimum(np.array(lens), T)
+    g = torch.Generator(device=dev).manual_seed(n)
+    idx = torch.randint(0, 99, (n, T + 3), device=dev, generator=g)[:, 1:T + 1]
+    starts, rows = torch.from_numpy(T - lens).to(dev), torch.randperm(n, device=dev, generator=g)
+    M = int(lens.sum())
+    out = torch.full((4, max(M, 1)), -1, dtype=torch.int64, device=dev)
+    cu = torch.full((2, n + 1), -1, dtype=torch.int32, device=dev)
+    _lib.check(_lib.lib().uv_pack_prompts(idx.data_ptr(), idx.stride(0), T, starts.data_ptr(), rows.data_ptr(), n, M,
+                                          cu[0].data_ptr(), cu[1].data_ptr(), *(o.data_ptr() for o in out),
+                                          stream_ptr(out.device)), "uv_pack_prompts")
+    want = pack_prompts(idx, starts, rows, lens)
+    assert torch.equal(cu[0], want["cu"]) and torch.equal(cu[1], want["tile_cu"])
+    for got, name in zip(out, ("tok", "pos", "rows", "last_pos")):
+        assert torch.equal(got[:M], want[name])
+    for dtype in (torch.float16, torch.bfloat16):
+        x = torch.randn(max(M, 1), 72, device=dev, generator=g).to(dtype)
+        y = torch.empty(n, 72, dtype=dtype, device=dev)
+        _lib.check(_lib.lib().uv_gather_norm(x.data_ptr(), 1 if dtype == torch.float16 else 2, 72, cu[0].data_ptr(), n,
+                                             y.data_ptr(), stream_ptr(x.device)), "uv_gather_norm")
+        ref = torch.nn.functional.rms_norm(x.float(), (72,))[want["last_row"]].masked_fill(want["empty"][:, None], 0)
+        assert torch.allclose(y.float(), ref, rtol=1e-2, atol=1e-3)
+
+
+@pytest.mark.parametrize("shape", [(1, 3), (7, 16384), (3, 1003)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_softcap(shape, dtype):
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.kernels._util import DTYPE_CODE, stream_ptr
+    x = (torch.randn(shape, device="cuda") * 20).to(dtype)
+    out = torch.empty(shape, device="cuda")
+    _lib.check(_lib.lib().uv_softcap(x.data_ptr(), DTYPE_CODE[dtype], x.numel(), 23.0, 5.0, 7.5, out.data_ptr(),
+                                     stream_ptr(x.device)), "uv_softcap")
+    assert torch.allclose(out, 23.0 * torch.sigmoid((x.float() + 5.0) / 7.5), rtol=1e-5, atol=1e-6)

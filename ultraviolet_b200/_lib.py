@@ -17,6 +17,7 @@ UV_ABI_VERSION = 2
 
 _lock = threading.Lock()
 _lib = None
+_host = None
 
 
 class UvError(RuntimeError):
@@ -150,6 +151,10 @@ SIGNATURES = {
     "uv_gemm_resid_norm": (C.c_int, [C.c_void_p, C.c_int64, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p,
                                      C.c_void_p, C.c_int, C.c_int, C.c_int, C.c_void_p]),
     "uv_fuse_weights": (C.c_int, [C.POINTER(FuseArgs), C.c_void_p]),
+    "uv_pack_prompts": (C.c_int, [C.c_void_p, C.c_int64, C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int64]
+                        + [C.c_void_p] * 7),
+    "uv_gather_norm": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
+    "uv_softcap": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_void_p, C.c_void_p]),
     "uv_sched_step": (C.c_int, [C.POINTER(SchedArgs), C.c_void_p]),
     "uv_sched_admit": (C.c_int, [C.POINTER(SchedArgs), C.POINTER(SchedAdmitArgs), C.c_void_p]),
     "uv_sched_enqueue": (C.c_int, [C.POINTER(SchedArgs), C.c_int, C.c_void_p]),
@@ -181,6 +186,24 @@ def lib() -> C.CDLL:
                 raise UvError(f"libuvdecode ABI {h.uv_abi_version()} != binding {UV_ABI_VERSION}: rebuild")
             _lib = h
     return _lib
+
+
+def host():
+    """The native host module (_uvhost, built next to the library), bound to the loaded libuvdecode.so."""
+    global _host
+    if _host is None:
+        lib()
+        with _lock:
+            if _host is None:
+                import torch  # noqa: F401  (its libraries are what the module links against)
+                try:
+                    from . import _uvhost
+                except ImportError as e:
+                    raise UvError(f"the _uvhost module cannot be loaded ({e}): build it with `python -m "
+                                  "ultraviolet_b200.build`") from e
+                _uvhost.init(LIB_PATH, UvError)
+                _host = _uvhost
+    return _host
 
 
 def check(code: int, what: str) -> None:

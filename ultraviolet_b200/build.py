@@ -16,6 +16,8 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libuvdecode.so")
+HOST_SRC = os.path.join(CSRC, "host.cpp")
+HOST_LIB = os.path.join(HERE, "_uvhost.so")
 OBJ_DIR = os.path.join(HERE, "build")
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH_FLAGS + ["-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC",
@@ -70,7 +72,29 @@ def build(force: bool = False, verbose: bool = False) -> str:
         r = subprocess.run([nvcc] + ARCH_FLAGS + ["-shared", "-o", LIB] + objs, capture_output=True, text=True)
         if r.returncode:
             raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    build_host(force)
     return LIB
+
+
+def build_host(force: bool = False) -> str:
+    """Compile csrc/host.cpp, the host-side extension module, against the installed torch."""
+    if not force and not _stale(HOST_LIB, [HOST_SRC, os.path.join(os.path.dirname(HERE), "include", "uvdecode.h")]):
+        return HOST_LIB
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(nvcc_path())))
+    inc = [os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = (["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-DTORCH_API_INCLUDE_EXTENSION_H",
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + ["-isystem" + i for i in inc]
+           + [HOST_SRC, "-o", HOST_LIB, "-L" + os.path.join(base, "lib"), "-L" + os.path.join(cuda, "lib64"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+              "-ltorch_cuda", "-ltorch", "-ltorch_python", "-lcublas", "-ldl"])
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode:
+        raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    return HOST_LIB
 
 
 if __name__ == "__main__":

@@ -73,6 +73,7 @@ class DecodeEngine:
         if cfg.rope_pairs:
             self.inv_freq.copy_((1.0 / cfg.rope_base) ** torch.linspace(0, 1, cfg.rope_pairs, dtype=torch.float32))
         self._scratch: dict[int, dict] = {}
+        self._prefill_trunk = None
         self._fuse_plan = None      # load_from's launch arguments for the parameter tensors it saw last
         self._fuse_status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.version = 0
@@ -572,9 +573,32 @@ class DecodeEngine:
 
     def logits(self, h: Tensor) -> Tensor:
         """MathLM.logits (model.py:824-827): fp32 softcapped logits, for API callers that want the full matrix."""
-        a, b, c = self.cfg.softcap
-        z = torch.mm(h.to(self.dtype), self.w["embed"].t()).float()
-        return a * torch.sigmoid((z + b) / c)
+        return self.softcap(torch.mm(h.to(self.dtype), self.w["embed"].t()))
+
+    def softcap(self, head: Tensor) -> Tensor:
+        """fp32 softcapped logits of raw (B, V) head output."""
+        out = torch.empty(head.shape, dtype=torch.float32, device=head.device)
+        with torch.cuda.device(self.device):
+            _lib.check(_lib.lib().uv_softcap(head.data_ptr(), DTYPE_CODE[head.dtype], head.numel(), *self.cfg.softcap,
+                                             out.data_ptr(), stream_ptr(self.device)), "uv_softcap")
+        return out
+
+    def prefill_trunk(self):
+        """The native host loop of a packed prompt pass (None: this engine runs its trunk another way)."""
+        if not self.fold or self.sw_qkv != "0" or not self.rope_table:
+            return None
+        if self._prefill_trunk is None:
+            cfg, w, L = self.cfg, self.w, range(self.cfg.n_layers)
+            ptr = lambda t: 0 if t is None else t.data_ptr()
+            per = lambda n: [w[f"l{l}.{n}"] for l in L]
+            self._prefill_trunk = _lib.host().PrefillTrunk(
+                per("wqkv"), per("wo"), per("gu"), per("down"), [ptr(w.get(f"l{l}.ve_gate")) for l in L],
+                [ptr(w.get(f"l{l}.attn_gate")) for l in L], [ptr(self.xsa[l]) if cfg.xsa else 0 for l in L],
+                [not cfg.is_global(l) for l in L], [(not cfg.is_global(l)) or cfg.global_rope for l in L],
+                [0 if cfg.is_global(l) else cfg.window for l in L], w["embed"], w.get("value_embed"), self.inv_freq,
+                cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, cfg.d_ff, cfg.rope_pairs, cfg.gate_channels,
+                cfg.ve_gate_channels, cfg.attn_scale, cfg.xsa_eps)
+        return self._prefill_trunk
 
     def sample(self, head: Tensor, temperature: float, top_p: float = 1.0, u: Tensor | None = None, seed: int = 0,
                row_keys: Tensor | None = None, steps: Tensor | None = None, tok_out: Tensor | None = None,

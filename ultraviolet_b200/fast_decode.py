@@ -110,8 +110,9 @@ def prefill_fast(self, idx: Tensor, starts: Tensor, st: KernelDecodeState, rows:
         rows = torch.arange(n, device=dev)
     rows = rows.to(torch.int64)
     starts = starts.to(torch.int64).contiguous()
-    lens_h = (T - starts).clamp_(min=0).cpu().numpy()   # the one host round trip (the reference has one too, :111)
-    hfin = torch.zeros(n, eng.cfg.d_model, dtype=eng.dtype, device=dev)
+    # the one host round trip (the reference has one too, :111)
+    lens_h = np.clip(T - starts.cpu().numpy(), 0, T)
+    hfin = None
     # passes over whole prompts, at most PREFILL_CHUNK_TOKENS packed rows each (one prompt alone may exceed it)
     a = 0
     while a < n:
@@ -119,13 +120,22 @@ def prefill_fast(self, idx: Tensor, starts: Tensor, st: KernelDecodeState, rows:
         while b < n and (b == a or tot + int(lens_h[b]) <= PREFILL_CHUNK_TOKENS):
             tot += int(lens_h[b])
             b += 1
-        if tot > 0:
+        if tot > 0 and b - a == n:
+            hfin = prefill_packed(eng, st, idx, starts, rows, lens_h)
+        elif tot > 0:
+            if hfin is None:
+                hfin = torch.zeros(n, eng.cfg.d_model, dtype=eng.dtype, device=dev)
             hfin[a:b] = prefill_packed(eng, st, idx[a:b], starts[a:b], rows[a:b], lens_h[a:b])
         a = b
-    st.starts[rows] = starts
-    st.pos[rows] = T
-    st.host_pos[rows.cpu().numpy()] = T
-    return eng.logits(hfin)
+    if full:
+        st.starts.copy_(starts)
+        st.pos.fill_(T)
+        st.host_pos[:] = T
+    else:
+        st.starts[rows] = starts
+        st.pos[rows] = T
+        st.host_pos[rows.cpu().numpy()] = T
+    return eng.logits(torch.zeros(n, eng.cfg.d_model, dtype=eng.dtype, device=dev) if hfin is None else hfin)
 
 
 def pack_prompts(idx: Tensor, starts: Tensor, rows: Tensor, lens_h) -> dict:
@@ -151,7 +161,15 @@ def pack_prompts(idx: Tensor, starts: Tensor, rows: Tensor, lens_h) -> dict:
 
 def prefill_packed(eng, st, idx: Tensor, starts: Tensor, rows: Tensor, lens_h) -> Tensor:
     """One packed pass: returns the final normed hidden state of every prompt's last token (n, d) (zeros for an
-    empty prompt)."""
+    empty prompt).  The packing, the launches and the library calls of the pass are issued by the native host loop
+    (some 75 of them cost more from Python than they run for at a few dozen tokens)."""
+    trunk = eng.prefill_trunk()
+    if trunk is not None and idx.dtype == torch.int64 and idx.stride(1) == 1:
+        lens = np.asarray(lens_h, dtype=np.int64)
+        M = int(lens.sum())
+        s = eng.scratch(M)
+        return trunk.run(idx, starts, rows, M, int(((lens + 15) // 16).sum()), s["x"], s["xn"], s["qkv"], s["z"], s["gu"],
+                         s["act"], s["gate"], s["rope_cs"], s["oob"], st.k, st.v, st.k_scale, st.v_scale)
     pk = pack_prompts(idx, starts, rows, lens_h)
     zero = torch.zeros(pk["M"], dtype=torch.int64, device=idx.device)
     h = eng.trunk(pk["tok"], st, pk["pos"], zero, g_len=idx.size(1), row_map=pk["rows"], packed=pk)

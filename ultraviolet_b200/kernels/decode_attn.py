@@ -137,8 +137,17 @@ def decode_attention(q: Tensor, k_cache: Tensor, v_cache: Tensor, pos: Tensor, s
     k_scale / v_scale (B, K, S) fp16; pos (B,) = position of the newest key (already written); keys attended are
     positions max(starts[b], pos[b] - window + 1, 0) .. pos[b]; ring: slot of position t is t % S (default:
     window > 0).  block_n / num_warps / backend are accepted and ignored (one kernel, fixed 128-key tiles).
-    Registered as the torch custom op ``uvb200::decode_attn`` (opaque to torch.compile, graph-capturable).
+    Registered as the torch custom op ``uvb200::decode_attn`` (opaque to torch.compile, graph-capturable); a plain eager
+    call on tensors as a cache holds them skips the op's dispatch and goes through the native host path, which takes
+    8 us of host time instead of 45.
     """
+    if (not torch.compiler.is_compiling() and k_scale is not None and v_scale is not None
+            and isinstance(pos, Tensor) and isinstance(starts, Tensor)):
+        out = _lib.host().decode_attention(q, k_cache, v_cache, pos, starts, scale, window,
+                                           -1 if ring is None else int(bool(ring)), k_scale, v_scale, ctx_hint or 0,
+                                           -2 ** 31 if num_splits is None else num_splits)
+        if out is not None:
+            return out
     if q.dim() == 4:
         q = q.reshape(q.size(0), q.size(-2), q.size(-1))
     need_cuda(q, k_cache, v_cache, pos, starts, k_scale, v_scale)

@@ -22,6 +22,10 @@ def fused_sample(x: Tensor, u: Tensor, softcap, temperature: float = 1.0, block:
                  top_p: float = 1.0) -> tuple[Tensor, Tensor]:
     """x (B, V) raw head output (before the softcap), u (B,) fp32 uniforms in [0, 1) -> (tokens int64 (B,),
     log softmax(softcap(x) / T)[token] fp32 (B,)).  Graph-capturable; `block` is accepted and ignored."""
+    if not torch.compiler.is_compiling() and isinstance(u, Tensor):
+        got = _lib.host().fused_sample(x, u, *map(float, softcap), float(temperature), float(top_p))
+        if got is not None:
+            return got
     need_cuda(x, u)
     B, V = x.shape
     if x.stride(1) != 1:
