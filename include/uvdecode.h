@@ -488,6 +488,48 @@ int uv_gather_norm(const void* x, int dtype, int d, const int32_t* cu, int n, vo
 /* out = a * sigmoid((x + b) / c), fp32, of the (B, V) raw head output (MathLM.logits, ultraviolet/model.py:824-827). */
 int uv_softcap(const void* x, int dtype, int64_t n, float a, float b, float c, float* out, void* stream);
 
+/* ---------------------------------------------------------------------------------------------------------------
+ * All transformer layers of one decode step of a small batch as ONE launch: embedding + norm, then per layer QKV projection, QK norm /
+ * RoPE / value-embedding gate, int8 append, attention (XSA + head gate), output projection, SwiGLU MLP, and the final
+ * norm (decode_step_fast without the head, ultraviolet/kernels/fast_decode.py:272-334), on the folded residual stream:
+ * wo and down carry the residual lambdas, norms are applied by the consumer.  A cooperative launch: one CTA
+ * per multiprocessor, which hand activations to each other through `workspace` (uv_decode_step_workspace_bytes,
+ * initialised by the call).  xn (B, d) is the result.  Batch entries must not read cache entries that another entry of
+ * the same call writes.  status: bit 3 is set when a CTA waited too long for another one.
+ *
+ * uv_decode_step_supported: 1 when the shapes and the current device allow uv_decode_step (head_dim 64, one KV head, at
+ * most 8 query heads, d and f multiples of 64, d at most 1024, local rings of at least 32 slots, at most 16 layers,
+ * at most 48 batch entries, one 8-wide tile of the QKV, output and down projections and two of gate and up per
+ * multiprocessor), else 0.
+ */
+typedef struct {
+  const void *wqkv, *wo, *gu, *down;   /* (N, K) row-major weights of the layer */
+  const void *ve_gate;                 /* (1, ve_ch) or NULL */
+  const void *attn_gate;               /* (H, gate_ch) or NULL */
+  const float* xsa_alpha;              /* (H,) or NULL */
+  int8_t *k_cache, *v_cache;
+  uint16_t *k_scale, *v_scale;
+  int S, S_alloc, ring, window, rope, reserved_;
+} uv_step_layer;
+
+typedef struct {
+  int dtype, B, n_layers, d, H, K, hd, f;
+  int64_t vocab;
+  const int64_t *tok, *pos, *starts, *row_map;
+  const void *embed, *value_embed;
+  const float* inv_freq;
+  int n_pairs, gate_ch, ve_ch;
+  float scale, xsa_eps;
+  void *xn, *workspace;
+  size_t workspace_bytes;
+  int *oob_count, *status;
+  const uv_step_layer* h_layers;       /* host array of n_layers entries, copied into the launch */
+} uv_step_args;
+
+int uv_decode_step(const uv_step_args* a, void* stream);
+int uv_decode_step_supported(const uv_step_args* a);
+size_t uv_decode_step_workspace_bytes(const uv_step_args* a);
+
 #ifdef __cplusplus
 }
 #endif

@@ -83,6 +83,24 @@ class FuseArgs(C.Structure):
                [("h_layers", C.POINTER(FuseLayer))]
 
 
+class StepLayer(C.Structure):
+    """uv_step_layer (include/uvdecode.h)."""
+    _fields_ = [(n, C.c_void_p) for n in ("wqkv", "wo", "gu", "down", "ve_gate", "attn_gate", "xsa_alpha", "k_cache",
+                                          "v_cache", "k_scale", "v_scale")] + \
+               [(n, C.c_int) for n in ("S", "S_alloc", "ring", "window", "rope", "reserved_")]
+
+
+class StepArgs(C.Structure):
+    """uv_step_args (include/uvdecode.h)."""
+    _fields_ = [(n, C.c_int) for n in ("dtype", "B", "n_layers", "d", "H", "K", "hd", "f")] + [("vocab", C.c_int64)] + \
+               [(n, C.c_void_p) for n in ("tok", "pos", "starts", "row_map", "embed", "value_embed", "inv_freq")] + \
+               [("n_pairs", C.c_int), ("gate_ch", C.c_int), ("ve_ch", C.c_int), ("scale", C.c_float),
+                ("xsa_eps", C.c_float)] + \
+               [("xn", C.c_void_p), ("workspace", C.c_void_p), ("workspace_bytes", C.c_size_t), ("oob_count", C.c_void_p),
+                ("status", C.c_void_p)] + \
+               [("h_layers", C.POINTER(StepLayer))]
+
+
 class SchedArgs(C.Structure):
     _fields_ = [(n, C.c_void_p) for n in (
         "req", "fed", "gen", "cur_tok", "pos", "starts", "row_key", "step_ctr", "samp_tok", "samp_lp", "prompt_off",
@@ -155,6 +173,9 @@ SIGNATURES = {
                         + [C.c_void_p] * 7),
     "uv_gather_norm": (C.c_int, [C.c_void_p, C.c_int, C.c_int, C.c_void_p, C.c_int, C.c_void_p, C.c_void_p]),
     "uv_softcap": (C.c_int, [C.c_void_p, C.c_int, C.c_int64, C.c_float, C.c_float, C.c_float, C.c_void_p, C.c_void_p]),
+    "uv_decode_step": (C.c_int, [C.POINTER(StepArgs), C.c_void_p]),
+    "uv_decode_step_supported": (C.c_int, [C.POINTER(StepArgs)]),
+    "uv_decode_step_workspace_bytes": (C.c_size_t, [C.POINTER(StepArgs)]),
     "uv_sched_step": (C.c_int, [C.POINTER(SchedArgs), C.c_void_p]),
     "uv_sched_admit": (C.c_int, [C.POINTER(SchedArgs), C.POINTER(SchedAdmitArgs), C.c_void_p]),
     "uv_sched_enqueue": (C.c_int, [C.POINTER(SchedArgs), C.c_int, C.c_void_p]),

@@ -117,6 +117,9 @@ class DecodeEngine:
         self.sw_qkv = os.environ.get("UVDECODE_SW_QKV", "0")
         if not (self.fold and self.tc_gemm_ok and d // 64 <= 12):
             self.sw_qkv = "0"
+        # The folded step's layers as ONE launch (uv_decode_step), wherever the library takes the shapes (small batches).
+        # UVDECODE_STEP=0: one launch per operation.
+        self.one_launch = self.fold and self.sw_qkv == "0" and os.environ.get("UVDECODE_STEP", "1") != "0"
         self.n_sm = torch.cuda.get_device_properties(self.device).multi_processor_count
         _lib.lib()
 
@@ -269,7 +272,7 @@ class DecodeEngine:
                      ss_x=torch.zeros(max(d // 128, 1), B, dtype=torch.float32, device=dev),
                      ss_h=torch.zeros(max(d // 128, 1), B, dtype=torch.float32, device=dev))
             # device words the kernels raise on silent failures: [0] attention status (bit 0: a bulk copy did not
-            # land in time, outputs of that launch are undefined), [1] count of skipped out-of-range KV writes
+            # land in time, bit 3: a wait of uv_decode_step ran out; outputs of that launch are undefined), [1] count of skipped out-of-range KV writes
             s["status"], s["oob"] = s["flags"][0:1], s["flags"][1:2]
             self._scratch[key] = s
         return s
@@ -293,12 +296,13 @@ class DecodeEngine:
                 if B is None or b == B or (isinstance(b, tuple) and b[0] == B):
                     s["flags"].zero_()
             raise _lib.UvError(f"decode kernels reported a device-side failure: attention status word "
-                               f"{d['attn_status']:#x} (bit 0 = a cache tile copy timed out), {d['kv_oob']} KV "
+                               f"{d['attn_status']:#x} (bit 0 = a cache tile copy timed out, bit 3 = a wait inside the one-launch step), {d['kv_oob']} KV "
                                "cache writes skipped as out of range; tokens produced since the last check are invalid")
         return d
 
     def launches_per_step(self) -> int:
-        """Kernel launches of one trunk + head call (the sampler is one more)."""
+        """Kernel launches of one trunk + head call (the sampler is one more).  A batch that uv_decode_step takes has one
+        launch for all layers."""
         n = self.cfg.n_layers
         if self.tc_gemm:
             return 1 + 5 * n + 2
@@ -320,7 +324,7 @@ class DecodeEngine:
     # ------------------------------------------------------------------------------------------------ one step
     def trunk(self, tok: Tensor, st, pos: Tensor, starts: Tensor, g_len: int | None = None,
               num_splits: dict | None = None, row_map: Tensor | None = None, skip_attn: bool = False,
-              packed: dict | None = None, scratch_tag: str = "") -> Tensor:
+              packed: dict | None = None, scratch_tag: str = "", shared_rows: bool = False) -> Tensor:
         """One token for every batch entry: writes K/V at `pos` and returns the final normed hidden (B, d) (a view
         of engine scratch, overwritten by the next call).  pos/starts are batch-indexed (B,) int64; row_map
         optionally maps batch entries to cache rows.
@@ -329,7 +333,10 @@ class DecodeEngine:
         dict(cu=int32 (n + 1,) first row of each prompt, tile_cu=int32 (n + 1,) first 16-token tile of each prompt,
         n_seq, max_tiles, last_pos=int64 (B,) last position of the entry's prompt).  Attention then runs over the
         unquantised keys / values of the batch itself (uv_prefill_attn) instead of the cache, and ring caches keep
-        only the newest positions of each prompt."""
+        only the newest positions of each prompt.
+
+        shared_rows: several entries of this call may be tokens of one sequence and read each other's keys (prefill
+        lanes): every layer's append then has to finish before its attention starts."""
         cfg, lib, dt = self.cfg, _lib.lib(), DTYPE_CODE[self.dtype]
         B = tok.size(0)
         s = self.scratch(B, scratch_tag)
@@ -341,6 +348,17 @@ class DecodeEngine:
         fused = self.fused_gemm and packed is None
         qkv_in_attn = self.qkv_in_attn and packed is None
         fold = self.fold
+        if self.one_launch and packed is None and not skip_attn and not shared_rows and not ns:
+            with torch.cuda.device(self.device):
+                a = self._step_args(tok, st, pos, starts, rm, s)
+                if lib.uv_decode_step_supported(C.byref(a)):
+                    ws = s.get("step_ws")
+                    if ws is None:
+                        n = lib.uv_decode_step_workspace_bytes(C.byref(a))
+                        ws = s["step_ws"] = torch.empty(n, dtype=torch.uint8, device=self.device)
+                    a.workspace, a.workspace_bytes = ws.data_ptr(), ws.numel()
+                    _lib.check(lib.uv_decode_step(C.byref(a), sp), "uv_decode_step")
+                    return s["xn"]
         if self.tc_gemm and not fused and not qkv_in_attn and B <= self.BIG_ROWS:
             return self._trunk_tc(tok, st, pos, starts, g_len, ns, rm, row_map, skip_attn, packed)
         with torch.cuda.device(self.device):
@@ -455,6 +473,31 @@ class DecodeEngine:
                 _lib.check(lib.uv_resid_norm(x.data_ptr(), x.data_ptr(), self._unit_lambdas().data_ptr(), dt, d,
                                              h.data_ptr(), xn.data_ptr(), B, sp), "uv_resid_norm")
         return xn  # rms_norm of the last residual stream == the final norm (fast_decode.py:332-334)
+
+    def _step_args(self, tok, st, pos, starts, rm, s) -> "_lib.StepArgs":
+        """uv_step_args of one decode step on state st with the scratch set s."""
+        cfg, w, a = self.cfg, self.w, _lib.StepArgs()
+        layers = (_lib.StepLayer * cfg.n_layers)()
+        for l, y in enumerate(layers):
+            glob = cfg.is_global(l)
+            kc = st.k[l]
+            y.wqkv, y.wo, y.gu, y.down = (w[f"l{l}.{n}"].data_ptr() for n in ("wqkv", "wo", "gu", "down"))
+            y.ve_gate = w[f"l{l}.ve_gate"].data_ptr() if cfg.has_ve(l) else None
+            y.attn_gate = w[f"l{l}.attn_gate"].data_ptr() if cfg.gate_channels else None
+            y.xsa_alpha = self.xsa[l].data_ptr() if cfg.xsa else None
+            y.k_cache, y.v_cache = kc.data_ptr(), st.v[l].data_ptr()
+            y.k_scale, y.v_scale = st.k_scale[l].data_ptr(), st.v_scale[l].data_ptr()
+            y.S, y.S_alloc, y.ring = kc.size(2), kc.stride(1) // cfg.head_dim, int(not glob)
+            y.window = 0 if glob else cfg.window
+            y.rope = int(((not glob) or cfg.global_rope) and cfg.rope_pairs > 0)
+        a.dtype, a.B, a.n_layers, a.d, a.f = DTYPE_CODE[self.dtype], tok.size(0), cfg.n_layers, cfg.d_model, cfg.d_ff
+        a.H, a.K, a.hd, a.vocab = cfg.n_heads, cfg.n_kv_heads, cfg.head_dim, cfg.vocab_size
+        a.tok, a.pos, a.starts, a.row_map = tok.data_ptr(), pos.data_ptr(), starts.data_ptr(), rm
+        a.embed, a.value_embed = w["embed"].data_ptr(), w["value_embed"].data_ptr() if self.use_ve else None
+        a.inv_freq, a.n_pairs = self.inv_freq.data_ptr(), cfg.rope_pairs
+        a.gate_ch, a.ve_ch, a.scale, a.xsa_eps = cfg.gate_channels, cfg.ve_gate_channels, cfg.attn_scale, cfg.xsa_eps
+        a.xn, a.oob_count, a.status, a.h_layers = s["xn"].data_ptr(), s["oob"].data_ptr(), s["status"].data_ptr(), layers
+        return a
 
     def _trunk_tc(self, tok, st, pos, starts, g_len, ns, rm, row_map, skip_attn, packed) -> Tensor:
         """The step on the tensor-core GEMM path: per layer  uv_gemm_sw_qkv -> attention -> uv_gemm_sw_resid (wo) ->

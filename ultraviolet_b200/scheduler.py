@@ -240,7 +240,7 @@ class GpuScheduler:
         n = self.B if n is None else n
         if self.L > 0:
             h = eng.trunk(self.cur_tok, st, self.pos_all, self.starts_all, g_len=st.max_len,
-                          num_splits=self.num_splits, row_map=self.row_map)[:self.B]  # only slots are sampled
+                          num_splits=self.num_splits, row_map=self.row_map, shared_rows=True)[:self.B]  # only slots are sampled
         else:
             h = eng.trunk(self.cur_tok[:n], st, st.pos[:n], st.starts[:n], g_len=st.max_len,
                           num_splits=self.num_splits, row_map=self.step_row[:n] if self.packed else None)
