@@ -38,7 +38,7 @@ SMALL = dict(vocab_size=300, d_model=128, n_layers=3, d_ff=192, global_every=2, 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("B,max_len,over", [
-    (1, 300, {}), (8, 700, {}), (9, 130, {}), (16, 300, {}), (17, 530, {}), (48, 400, {}),
+    (1, 300, {}), (8, 700, {}), (9, 130, {}), (16, 300, {}), (17, 530, {}), (32, 400, {}), (48, 400, {}),
     (3, 90, SMALL), (33, 200, dict(SMALL, n_heads=3, xsa=False)), (2, 60, dict(SMALL, d_model=64, d_ff=64, n_heads=1)),
     (5, 100, dict(SMALL, attn_gate_channels=18, ve_gate_channels=5, window=33)),
     (7, 100, dict(SMALL, d_model=1024, d_ff=2048, n_layers=2))])

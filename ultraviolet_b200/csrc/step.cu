@@ -2,13 +2,15 @@
 //
 // What bounds a step: with a few rows every kernel of a layer is a 3-5 us chain of dependent round trips on a mostly idle
 // GPU, and 70 of them in a row took 255-310 us at 1-48 rows, against 17 us of weight traffic.  Here a layer is six hops
-// between CTAs of 0.6-1.2 us each with 0.3-0.5 us of work in between (the attention: 2.3 us): 100 us at 1 row, 144 at 16,
-// 202 at 32, 258 at 48 (UV-50M, contexts of 200-900).
+// between CTAs of 0.6-1.2 us each with 0.3-0.5 us of work in between (the attention: 2.3 us), and from some 16 rows on the
+// L2 traffic of CTAs that all read all rows: 100 us at 1 row, 110 at 8, 143 at 16, 175 at 32, 209 at 48 (UV-50M, contexts of
+// 200-900).
 //
 // Split: one CTA per multiprocessor.  In the projections a CTA owns one 8-wide tile of output features (of gate | up up to
 // two pairs of tiles; UV-50M has 80, 80, 208 pairs and 80) for all rows, its weights in shared memory, fetched a layer
-// ahead (the region of a phase is refilled as soon as the phase has used it).  The 16 warps are slices of K, whose sums
-// meet in shared memory; row tiles of 16 follow one another.  In the attention phase the last CTAs own a row each, a warp
+// ahead (the region of a phase is refilled as soon as the phase has used it).  The 16 warps are row tiles
+// of 16 times slices of K, whose sums meet in shared memory (with the tiles one after the other, 16 slices each, 32 rows took
+// 202 us and 48 took 258).  In the attention phase the last CTAs own a row each, a warp
 // per head for what is done head by head, chunks of keys dealt out to the warps in between.
 //
 // Exchange: activations change hands through L2 without barriers, fences or flags on the way.  The workspace starts out
@@ -20,7 +22,7 @@
 // Matrix instructions: warp-level mma.sync, because operands go from L2 to registers and results from registers to L2 in
 // the phase's critical path of a few hundred cycles.  tcgen05 with its TMA tiles, commits and TMEM reads cost 2-3 thousand
 // cycles a phase at these sizes (23 us a layer at one row against 10 here).  What counts is the number of instructions on
-// the path of a warp: about six cycles each.  Hence one row tile at a time with fixed tile counts, sums of squares out of
+// the path of a warp: about six cycles each.  Hence fixed tile counts, sums of squares out of
 // the tensor cores, and a code size that the instruction caches hold.
 //
 // Attention: a warp takes 32-key chunks of one row straight from the cache into MMA fragments (whole 64-byte key rows, one
@@ -28,7 +30,7 @@
 // cache rows are prefetched to L2.  The entry at the row's own position is taken from shared memory.
 //
 // Rounding points are those of the per-kernel folded step (engine.py): projections round to the activation dtype, norms
-// scale the rounded projection, the residual stream rounds once per update.
+// scale the rounded projection, the residual stream adds it.
 //
 // Every wait is bounded (200 ms); a CTA that gives up sets status bit 3, skips its later waits and still ends.
 #include <mutex>
@@ -42,13 +44,14 @@ namespace uv {
 constexpr int ST_WARPS = 16;
 constexpr int ST_THREADS = ST_WARPS * 32;
 constexpr int ST_MAXL = 16;                 // layers per launch (kernel parameter space)
-// Rows of a batch: a row tile more costs 55 us here and 5 a step of single kernels, which win from 64 rows on (314 : 310 us;
-// 258 : 312 at 48).
+// Rows of a batch: at most three row tiles, which the 16 warps take side by side.  Past them the CTAs' reads of all rows and
+// the one CTA that a row has for its attention eat up the gain: 209 against 310 us at 48 rows, 232 : 309 at 64, 294 : 337 at 64
+// of 8192 keys, and from 65 on (two passes over the weights) 288 : 312, 320 : 315 at 96.
 constexpr int ST_ROWS = 48;
 constexpr int ST_XCH = 128;                 // leading channels of a row that the gates may read
 constexpr int ST_HD = 64;
 constexpr int ST_PAIRS = 2;                 // 8-wide gate | up tile pairs a CTA can have (one tile of the other projections)
-constexpr unsigned ST_NAP = 40;              // ns between two looks for a missing word: the stores need the L2 too
+constexpr unsigned ST_NAP = 100;              // ns between two looks for a missing word: the stores need the L2 too
 constexpr uint32_t ST_EMPTY = 0xffffffffu;
 constexpr unsigned long long ST_WAIT_NS = 200ull * 1000ull * 1000ull;
 
@@ -119,7 +122,7 @@ template <typename T> __device__ __forceinline__ void st_scale8(float (&x)[8], f
 }
 
 
-template <typename T, int ROWS> struct StepSmem {
+template <typename T, int ROWS, int LGM> struct StepSmem {
   alignas(16) T vcur[ST_HD];              // unquantised value of the owned row's token
   float vinv2;                            // 1 / |it|^2
   alignas(16) int8_t qi[2][8][ST_HD];     // its query heads in two int8 parts (split_q, attn_math.cuh)
@@ -127,8 +130,10 @@ template <typename T, int ROWS> struct StepSmem {
   alignas(16) int8_t q8[2][ST_HD];        // its quantised key and value
   uint16_t sc[2];
   alignas(16) StepLayerK layer[ST_MAXL];  // (from the constant bank every first touch of a layer costs ~500 cycles)
-  alignas(16) uint32_t xs[ST_ROWS][4];    // this CTA's tile of the residual stream
-  alignas(16) float2 red[2][(2 * ST_PAIRS + 1) * ROWS * 4 * (ST_WARPS + 2)];   // partial sums
+  // partial sums: [tile][row][feature pair][slice of K], rows of 2^LGM row tiles; their sums of squares: [row][slice]
+  static constexpr int MROWS = ROWS << LGM, KS = ST_WARPS >> LGM, LD = KS == 4 ? 4 : KS + 2, TILE = MROWS * 4 * LD;
+  alignas(16) float2 red[2][2 * ST_PAIRS * TILE];
+  alignas(16) float ssq[2][MROWS * KS];
   float mg_m[8][ST_WARPS], mg_l[8][ST_WARPS], mg_o[ST_WARPS][8][ST_HD];        // the attention's per-warp results
   uint64_t full[4];                       // weights of a phase have landed
   int dead;
@@ -337,41 +342,50 @@ __device__ __forceinline__ bool st_late(unsigned long long& t_begin, volatile in
   *dead = 1;
   return true;
 }
-// Load N pieces of 16 bytes until none holds an empty word (the largest unsigned one).  Warp-collective.
+// Load N pieces of 16 bytes until none holds an empty word (the largest unsigned one), again only what did.  Warp-collective.
 template <int N, typename At>
 __device__ __forceinline__ void st_take(uint4 (&u)[N], At at, volatile int* dead) {
   unsigned long long t_begin = 0;
+#pragma unroll
+  for (int j = 0; j < N; ++j) u[j] = st_peek(at(j));
 #pragma unroll 1
   for (int i = 0;; ++i) {
-    uint32_t top = 0u;
+    bool missing[N], any = false;
 #pragma unroll
-    for (int j = 0; j < N; ++j) u[j] = st_peek(at(j));
-#pragma unroll
-    for (int j = 0; j < N; ++j) top = max(max(top, max(u[j].x, u[j].y)), max(u[j].z, u[j].w));
-    if (!__any_sync(0xffffffffu, top == ST_EMPTY)) return;
-    __nanosleep(ST_NAP);
+    for (int j = 0; j < N; ++j) {
+      missing[j] = __any_sync(0xffffffffu, max(max(u[j].x, u[j].y), max(u[j].z, u[j].w)) == ST_EMPTY);
+      any |= missing[j];
+    }
+    if (!any) return;
     if ((i & 31) == 31 && __any_sync(0xffffffffu, st_late(t_begin, dead))) return;
+    __nanosleep(ST_NAP);
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+      if (missing[j]) u[j] = st_peek(at(j));
   }
 }
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
 // ------------------------------------------------------------------------------------------------ the kernel
 // HALF: at most 8 rows (the lower half of the MMA's 16; 110 us at 6 rows with it).
-template <typename T, bool HALF>
+template <typename T, bool HALF, int LGM>
 __global__ void __launch_bounds__(ST_THREADS, 1) step_kernel(const __grid_constant__ StepP P) {
   constexpr int ROWS = HALF ? 8 : 16, NR = HALF ? 1 : 2;
-  constexpr int LD = ST_WARPS + 2;                      // partial sums of a feature pair: float2 a warp, rows padded
-  constexpr int TILE = ROWS * 4 * LD;                   // float2 of a tile
+  // the warps are 2^LGM row tiles times KS slices of K
+  using Smem = StepSmem<T, ROWS, LGM>;
+  constexpr int MG = 1 << LGM, MROWS = Smem::MROWS, KS = Smem::KS, LD = Smem::LD, TILE = Smem::TILE;
+  constexpr int SL = KS / 4, FROWS = 8 / SL;            // threads a feature pair's sums take, rows of a warp there
   extern __shared__ __align__(128) unsigned char st_smem[];
-  StepSmem<T, ROWS>& sm = *reinterpret_cast<StepSmem<T, ROWS>*>(st_smem);
+  Smem& sm = *reinterpret_cast<Smem*>(st_smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rank = blockIdx.x, C = gridDim.x;
   const bool own = C - 1 - rank < P.B;                  // the last CTAs own a row each (the first ones have a tile of
   const int64_t orow = C - 1 - rank;                    // every projection)
   volatile int* const dead = &sm.dead;
   const int NQ = (P.H + 2) * ST_HD, NZ = P.H * ST_HD;
   const int r = lane >> 2, q = lane & 3;                // MMA fragment row and column pair
-  // finishing a projection: 16 threads a row of a tile (or pair), four of them for each pair of features
-  const int frow = (tid >> 4) & (ROWS - 1), ft = (tid >> 4) / ROWS, fq = (lane >> 2) & 3, sl = lane & 3;
+  // finishing a projection: SL threads for each pair of features of a row of a tile (or pair)
+  const int sl = tid & (SL - 1), fq = (tid / SL) & 3, frow = (tid / (4 * SL)) & (MROWS - 1), ft = tid / (4 * SL * MROWS);
+  const int mg = warp & (MG - 1), ks = warp >> LGM;
 
   // ---- weights of phase p, layer l into the phase's region: a bulk copy a row, dealt out over the warps (one issues some 25
   //      cycles apart, and would be late for the next phase with all of them)
@@ -505,100 +519,98 @@ __global__ void __launch_bounds__(ST_THREADS, 1) step_kernel(const __grid_consta
   if (own && warp == ST_WARPS - 1) prefetch_kv(0);
   // ---- the residual stream: two values of a row at the thread that finishes their sums
   const bool has_x = rank < P.rem[PH_WO] || P.base[PH_WO] > 0;
-  if (has_x && ft == 0)
-    for (int row = frow; (row & ~1) < P.B; row += ROWS) {
-      const uint32_t v = word(row < P.B ? ws + P.off[0] + rank * (ROWS * 8) + at_row(row, P.d) + 2 * fq : nullptr);
-      if (sl == 0 && row < P.B) sm.xs[row][fq] = v;
-    }
+  const bool fin = frow < P.B && sl == 0;
+  float2 res = make_float2(0.f, 0.f);
+  if (has_x && ft == 0 && (frow & ~(FROWS - 1)) < P.B)
+    res = st_unpack2<T>(word(frow < P.B ? ws + P.off[0] + rank * (ROWS * 8) + at_row(frow, P.d) + 2 * fq : nullptr));
 
   // ---- a projection: rows of `in` (row stride K) times this CTA's tiles of phase p; done(sums of this thread's pair of
   //      features (gate | up: of both), the row's norm factor (gate | up))
   int odd = 0;                                          // areas for partial sums take turns
   auto project = [&](auto phase, int l, const T* in, auto&& done) {
     constexpr int p = decltype(phase)::value, NT = p == PH_GU ? 2 * ST_PAIRS : 1;
-    constexpr int J = p == PH_DN ? 4 : 2;               // pieces of 32 K values in flight
+    // pieces of 32 K values in flight
+    constexpr int J = LGM == 0 ? (p == PH_DN ? 4 : 2) : LGM == 1 ? (p == PH_DN ? 4 : 3) : (p == PH_WO ? 4 : 5);
     const int mine = P.base[p] + (rank < P.rem[p]);     // tiles or pairs of this CTA: at most one, at most ST_PAIRS
     if (mine == 0) return;
     const int K = P.K[p], ld = 2 * K + 64;
-    const uint32_t w0 = smem_addr(st_smem + P.region[p]) + (uint32_t)(r * ld + warp * 64 + q * 16);
-    constexpr int PIECE = ST_WARPS * (p == PH_WO ? 32 : 32 * ROWS);   // elements between a warp's pieces
+    uint32_t w = smem_addr(st_smem + P.region[p]) + (uint32_t)(r * ld + ks * 64 + q * 16);
+    constexpr int PIECE = KS * (p == PH_WO ? 32 : 32 * ROWS);   // elements between a warp's pieces
     weights_ready(p, l);
+    // this lane's rows of the A fragments (past the batch: the last row again, whose sums nobody reads)
+    const int mt = mg * ROWS, ra = mt + r < P.B ? mt + r : P.B - 1, rb = mt + r + 8 < P.B ? mt + r + 8 : P.B - 1;
+    const int to_b = (rb - ra) * (p == PH_WO ? K : 8);
+    const T* pa = p == PH_WO ? in + ra * K + ks * 32 + 8 * q : in + (ks * 4 + q) * (ROWS * 8) + at_row(ra, K);
+    float2* const red = sm.red[odd];
+    float* const ssq = sm.ssq[odd];
+    odd ^= 1;
+    float acc[NT][4], gram[2][4];
+#pragma unroll
+    for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+#pragma unroll
+    for (int n = 0; n < 2; ++n) gram[n][0] = gram[n][1] = gram[n][2] = gram[n][3] = 0.f;
 #pragma unroll 1
-    for (int m0 = 0; m0 < P.B; m0 += ROWS) {
-      // this lane's rows of the A fragments (past the batch: the last row again, whose sums nobody reads)
-      const int ra = m0 + r < P.B ? m0 + r : P.B - 1, rb = m0 + r + 8 < P.B ? m0 + r + 8 : P.B - 1;
-      const int to_b = (rb - ra) * (p == PH_WO ? K : 8);
-      const T* pa = p == PH_WO ? in + ra * K + warp * 32 + 8 * q : in + (warp * 4 + q) * (ROWS * 8) + at_row(ra, K);
-      uint32_t w = w0;
-      float2* const red = sm.red[odd];                    // [tile][row][feature pair][warp]
-      odd ^= 1;
-      float acc[NT][4], gram[2][4];
+    for (int left = mt < P.B ? ((K >> 5) - ks + KS - 1) / KS : 0; left > 0; left -= J) {
+      uint4 u[J * NR];
+      st_take<J * NR>(u, [&](int j) { return pa + (j / NR < left ? (j / NR) * PIECE : 0) + (j % NR ? to_b : 0); }, dead);
 #pragma unroll
-      for (int n = 0; n < NT; ++n) acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f;
+      for (int j = 0; j < J; ++j)
+        if (j < left) {
+          const uint4 a = u[j * NR], b = HALF ? make_uint4(0u, 0u, 0u, 0u) : u[j * NR + NR - 1];
 #pragma unroll
-      for (int n = 0; n < 2; ++n) gram[n][0] = gram[n][1] = gram[n][2] = gram[n][3] = 0.f;
-#pragma unroll 1
-      for (int left = ((K >> 5) - warp + ST_WARPS - 1) / ST_WARPS; left > 0; left -= J) {
-        uint4 u[J * NR];
-        st_take<J * NR>(u, [&](int j) { return pa + (j / NR < left ? (j / NR) * PIECE : 0) + (j % NR ? to_b : 0); }, dead);
-#pragma unroll
-        for (int j = 0; j < J; ++j)
-          if (j < left) {
-            const uint4 a = u[j * NR], b = HALF ? make_uint4(0u, 0u, 0u, 0u) : u[j * NR + NR - 1];
-#pragma unroll
-            for (int n = 0; n < NT; ++n) {
-              uint4 b4;
-              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(b4.x), "=r"(b4.y), "=r"(b4.z), "=r"(b4.w)
-                           : "r"(w + (uint32_t)(n * 8 * ld + j * ST_WARPS * 64)));
-              st_mma<T>(acc[n], a.x, b.x, a.y, b.y, b4.x, b4.y);
-              st_mma<T>(acc[n], a.z, b.z, a.w, b.w, b4.z, b4.w);
-            }
-            if (p == PH_GU) {                             // sums of squares of the rows: the diagonal of rows times rows
-              st_mma<T>(gram[0], a.x, b.x, a.y, b.y, a.x, a.y);
-              st_mma<T>(gram[0], a.z, b.z, a.w, b.w, a.z, a.w);
-              if (!HALF) {
-                st_mma<T>(gram[1], a.x, b.x, a.y, b.y, b.x, b.y);
-                st_mma<T>(gram[1], a.z, b.z, a.w, b.w, b.z, b.w);
-              }
+          for (int n = 0; n < NT; ++n) {
+            if (MG > 1 && n > 1 && mine == 1) continue;
+            uint4 b4;
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(b4.x), "=r"(b4.y), "=r"(b4.z), "=r"(b4.w)
+                         : "r"(w + (uint32_t)(n * 8 * ld + j * KS * 64)));
+            st_mma<T>(acc[n], a.x, b.x, a.y, b.y, b4.x, b4.y);
+            st_mma<T>(acc[n], a.z, b.z, a.w, b.w, b4.z, b4.w);
+          }
+          if (p == PH_GU) {                             // sums of squares of the rows: the diagonal of rows times rows
+            st_mma<T>(gram[0], a.x, b.x, a.y, b.y, a.x, a.y);
+            st_mma<T>(gram[0], a.z, b.z, a.w, b.w, a.z, a.w);
+            if (!HALF) {
+              st_mma<T>(gram[1], a.x, b.x, a.y, b.y, b.x, b.y);
+              st_mma<T>(gram[1], a.z, b.z, a.w, b.w, b.z, b.w);
             }
           }
-        pa += J * PIECE, w += J * ST_WARPS * 64;
-      }
-      float2* at = red + lane * LD + warp;                // lane = row * 4 + pair
-#pragma unroll
-      for (int n = 0; n < NT; ++n) {
-        at[n * TILE] = make_float2(acc[n][0], acc[n][1]);
-        if (!HALF) at[n * TILE + 32 * LD] = make_float2(acc[n][2], acc[n][3]);
-      }
-      if (p == PH_GU) {
-        at[NT * TILE] = make_float2(gram[0][0], gram[0][1]);
-        if (!HALF) at[NT * TILE + 32 * LD] = make_float2(gram[1][2], gram[1][3]);
-      }
-      __syncthreads();
-      const int row = m0 + frow;
-      if (ft < mine && (row & ~1) < P.B) {                // (whole warps)
-        auto sum4 = [&](const float2* at) {               // of the four warps that are this thread's
-          const float4 x = reinterpret_cast<const float4*>(at)[0], y = reinterpret_cast<const float4*>(at)[1];
-          return make_float2((x.x + x.z) + (y.x + y.z), (x.y + x.w) + (y.y + y.w));
-        };
-        auto sum_quad = [](float2& v) {
-          v.x += __shfl_xor_sync(0xffffffffu, v.x, 1), v.y += __shfl_xor_sync(0xffffffffu, v.y, 1);
-          v.x += __shfl_xor_sync(0xffffffffu, v.x, 2), v.y += __shfl_xor_sync(0xffffffffu, v.y, 2);
-        };
-        const float2* from = red + (p == PH_GU ? 2 * ft * TILE : 0) + (frow * 4 + fq) * LD + 4 * sl;
-        float2 s0 = sum4(from), s1 = s0;
-        float ss = 0.f;
-        if (p == PH_GU) {
-          s1 = sum4(from + TILE);
-          const float2 g = sum4(red + NT * TILE + (frow * 4 + ((frow >> 1) & 3)) * LD + 4 * sl);
-          ss = frow & 1 ? g.y : g.x;
-          ss += __shfl_xor_sync(0xffffffffu, ss, 1);
-          ss += __shfl_xor_sync(0xffffffffu, ss, 2);
-          sum_quad(s1);
         }
-        sum_quad(s0);
-        done(row, s0, s1, p == PH_GU ? rsqrtf(ss / (float)P.d + RMS_EPS) : 0.f);
+      pa += J * PIECE, w += J * KS * 64;
+    }
+    float2* at = red + (mg * ROWS * 4 + lane) * LD + ks;  // lane = row * 4 + pair
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      at[n * TILE] = make_float2(acc[n][0], acc[n][1]);
+      if (!HALF) at[n * TILE + 32 * LD] = make_float2(acc[n][2], acc[n][3]);
+    }
+    if (p == PH_GU && q == (r >> 1)) {                  // columns 2 q, 2 q + 1
+      ssq[(mg * ROWS + r) * KS + ks] = r & 1 ? gram[0][1] : gram[0][0];
+      if (!HALF) ssq[(mg * ROWS + r + 8) * KS + ks] = r & 1 ? gram[1][3] : gram[1][2];
+    }
+    __syncthreads();
+    if (ft < mine && (frow & ~(FROWS - 1)) < P.B) {                // (whole warps)
+      auto sum4 = [&](const float2* at) {               // of the four slices that are this thread's
+        const float4 x = reinterpret_cast<const float4*>(at)[0], y = reinterpret_cast<const float4*>(at)[1];
+        return make_float2((x.x + x.z) + (y.x + y.z), (x.y + x.w) + (y.y + y.w));
+      };
+      auto sum_lanes = [](float2& v) {
+#pragma unroll
+        for (int o = 1; o < SL; o *= 2)
+          v.x += __shfl_xor_sync(0xffffffffu, v.x, o), v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+      };
+      const float2* from = red + (p == PH_GU ? 2 * ft * TILE : 0) + (frow * 4 + fq) * LD + 4 * sl;
+      float2 s0 = sum4(from), s1 = s0;
+      float ss = 0.f;
+      if (p == PH_GU) {
+        s1 = sum4(from + TILE);
+        const float4 g = *reinterpret_cast<const float4*>(ssq + frow * KS + 4 * sl);
+        ss = (g.x + g.y) + (g.z + g.w);
+#pragma unroll
+        for (int o = 1; o < SL; o *= 2) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        sum_lanes(s1);
       }
+      sum_lanes(s0);
+      done(s0, s1, p == PH_GU ? rsqrtf(ss / (float)P.d + RMS_EPS) : 0.f);
     }
     fetch(p, l + 1);                                    // (every warp is done with the weights)
   };
@@ -639,8 +651,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) step_kernel(const __grid_consta
       if (warp == ST_WARPS - 1 && l + 1 < P.L) prefetch_kv(l + 1);
     }
     // ---- QKV projection
-    project(std::integral_constant<int, PH_QKV>{}, l, x0, [&](int row, float2 a, float2, float) {
-      if (row < P.B && sl == 0) st_put(qkv + rank * (ROWS * 8) + at_row(row, NQ) + 2 * fq, st_word<T>(a.x, a.y));
+    project(std::integral_constant<int, PH_QKV>{}, l, x0, [&](float2 a, float2, float) {
+      if (fin) st_put(qkv + rank * (ROWS * 8) + at_row(frow, NQ) + 2 * fq, st_word<T>(a.x, a.y));
     });
     if (own) {
       // ---- the owned row, a warp a head (queries, key, value), two dimensions a lane: QK norm, RoPE, value embedding, int8
@@ -790,22 +802,20 @@ __global__ void __launch_bounds__(ST_THREADS, 1) step_kernel(const __grid_consta
     }
     // ---- output projection, gate | up, down
     auto residual = [&](T* out) {                       // x += sums
-      return [&, out](int row, float2 a, float2, float) {
-        if (row < P.B && sl == 0) {
-          const float2 x = st_unpack2<T>(sm.xs[row][fq]);
-          const uint32_t w = st_word<T>(x.x + a.x, x.y + a.y);
-          st_put(out + rank * (ROWS * 8) + at_row(row, P.d) + 2 * fq, w);
-          sm.xs[row][fq] = w;
-        }
+      return [&, out](float2 a, float2, float) {
+        a = st_rnd2<T>(a.x, a.y);
+        const uint32_t w = st_word<T>(res.x + a.x, res.y + a.y);
+        res = st_unpack2<T>(w);
+        if (fin) st_put(out + rank * (ROWS * 8) + at_row(frow, P.d) + 2 * fq, w);
       };
     };
     project(std::integral_constant<int, PH_WO>{}, l, zb, residual(x1));
-    project(std::integral_constant<int, PH_GU>{}, l, x1, [&](int row, float2 g, float2 u, float s) {
+    project(std::integral_constant<int, PH_GU>{}, l, x1, [&](float2 g, float2 u, float s) {
       float2 g2 = st_rnd2<T>(g.x, g.y), u2 = st_rnd2<T>(u.x, u.y);
       g2 = st_rnd2<T>(g2.x * s, g2.y * s), u2 = st_rnd2<T>(u2.x * s, u2.y * s);
       const float2 a = st_rnd2<T>(__fdividef(g2.x, 1.0f + __expf(-g2.x)), __fdividef(g2.y, 1.0f + __expf(-g2.y)));
-      if (row < P.B && sl == 0)
-        st_put(actb + (rank + ft * C) * (ROWS * 8) + at_row(row, P.f) + 2 * fq, st_word<T>(a.x * u2.x, a.y * u2.y));
+      if (fin)
+        st_put(actb + (rank + ft * C) * (ROWS * 8) + at_row(frow, P.f) + 2 * fq, st_word<T>(a.x * u2.x, a.y * u2.y));
     });
     project(std::integral_constant<int, PH_DN>{}, l, actb, residual(x0 + P.stride));
   }
@@ -833,9 +843,16 @@ __global__ void __launch_bounds__(ST_THREADS, 1) step_kernel(const __grid_consta
 constexpr size_t ST_SMEM_MAX = 227 * 1024;
 
 typedef void (*StepKernel)(const StepP);
-static StepKernel step_variant(bool f16, bool half) {
-  return f16 ? (half ? step_kernel<__half, true> : step_kernel<__half, false>)
-             : (half ? step_kernel<__nv_bfloat16, true> : step_kernel<__nv_bfloat16, false>);
+template <typename T> static StepKernel step_variant_of(int rows) {
+  return rows <= 8 ? step_kernel<T, true, 0> : rows <= 16 ? step_kernel<T, false, 0> : rows <= 32 ? step_kernel<T, false, 1>
+                                                                                                  : step_kernel<T, false, 2>;
+}
+static StepKernel step_variant(bool f16, int rows) {
+  return f16 ? step_variant_of<__half>(rows) : step_variant_of<__nv_bfloat16>(rows);
+}
+static size_t step_state_bytes(int rows) {
+  return rows <= 8 ? sizeof(StepSmem<__half, 8, 0>) : rows <= 16 ? sizeof(StepSmem<__half, 16, 0>)
+                   : rows <= 32 ? sizeof(StepSmem<__half, 16, 1>) : sizeof(StepSmem<__half, 16, 2>);
 }
 
 // Multiprocessors of the current device (0: it cannot run the kernel), asked for once per device.
@@ -851,8 +868,8 @@ static int step_sms() {
     int sms = 0, coop = 0;
     bool ok = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess &&
               cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop;
-    for (int k = 0; k < 4; ++k)
-      ok = ok && cudaFuncSetAttribute(step_variant(k & 1, k & 2), cudaFuncAttributeMaxDynamicSharedMemorySize,
+    for (int k = 0; k < 8; ++k)
+      ok = ok && cudaFuncSetAttribute(step_variant(k & 1, 8 << (k >> 1)), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       (int)ST_SMEM_MAX) == cudaSuccess;
     if (!ok) cudaGetLastError();
     known[dev] = ok ? sms : 0, done[dev] = true;
@@ -878,7 +895,7 @@ static bool step_plan(const uv_step_args* a, StepP* P, size_t* smem, int* sms) {
   P->B = a->B, P->L = a->n_layers, P->d = a->d, P->H = a->H, P->f = a->f;
   P->K[PH_QKV] = P->K[PH_GU] = a->d, P->K[PH_WO] = a->H * ST_HD, P->K[PH_DN] = a->f;
   const int tiles[4] = {(a->H + 2) * ST_HD / 8, a->d / 8, a->f / 8, a->d / 8};
-  size_t at = ((a->B <= 8 ? sizeof(StepSmem<__half, 8>) : sizeof(StepSmem<__half, 16>)) + 127) & ~(size_t)127;
+  size_t at = (step_state_bytes(a->B) + 127) & ~(size_t)127;
   for (int p = 0; p < 4; ++p) {
     const int most = p == PH_GU ? ST_PAIRS : 1;
     P->region[p] = (int)at;
@@ -954,7 +971,7 @@ extern "C" int uv_decode_step(const uv_step_args* a, void* stream) {
   attr[0].id = cudaLaunchAttributeCooperative;                   // its CTAs wait for one another: all of them or none
   attr[0].val.cooperative = 1;
   cfg.attrs = attr, cfg.numAttrs = 1;
-  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, step_variant(a->dtype == UV_F16, a->B <= 8), P);
+  if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, step_variant(a->dtype == UV_F16, a->B), P);
   if (e != cudaSuccess) {
     cudaGetLastError();
     set_last_cuda_error((int)e);
