@@ -98,39 +98,27 @@ __global__ void __launch_bounds__(512) prefill_attn_kernel(const __grid_constant
   pdl_wait();
   pdl_trigger();
 
-  // ---- which sequence / query tile: binary search of the tile prefix sums
-  const int tile = blockIdx.x;
-  if (tile >= P.tile_cu[P.n_seq]) return;
-  int lo_s = 0, hi_s = P.n_seq;  // invariant: tile_cu[lo_s] <= tile < tile_cu[hi_s]
-  while (hi_s - lo_s > 1) {
-    const int mid = (lo_s + hi_s) >> 1;
-    if (P.tile_cu[mid] <= tile) lo_s = mid;
-    else hi_s = mid;
-  }
-  const int seq = lo_s;
-  const int row0 = P.cu_seqlens[seq];
+  // ---- which sequence / query tile: the warp looks at 32 of the tile prefix sums at a time (two dependent loads for up to
+  //      1024 prompts).  With one at a time, Q fetched before the first key tile and the epilogue fetching V again, a launch
+  //      took 59 us at 256 prompts of 32 - 128 tokens (now 47), 72 at 7 of up to 2000 (66), 8.1 at one of 48 (6.8)
+  const int tile = blockIdx.x, n_tiles = P.tile_cu[P.n_seq];
+  int seq = 0, end = P.n_seq;  // tile_cu[seq] <= tile < tile_cu[end]
+  do {
+    const int step = (end - seq + 31) >> 5, at = seq + lane * step;
+    const bool below = at < end && P.tile_cu[at] <= tile;
+    const int n = __popc(__ballot_sync(0xffffffffu, below));  // (lane 0's is)
+    seq += (n > 0 ? n - 1 : 0) * step;
+    end = seq + step < end ? seq + step : end;
+  } while (end - seq > 1);
+  if (tile >= n_tiles) return;
+  const int row0 = P.cu_seqlens[seq], tile0 = P.tile_cu[seq];
   const int len = P.cu_seqlens[seq + 1] - row0;
-  const int q0 = (tile - P.tile_cu[seq]) * PF_QT;  // first query token (index inside the sequence)
+  const int q0 = (tile - tile0) * PF_QT;           // first query token (index inside the sequence)
   if (q0 >= len) return;
 
   const QT* base = static_cast<const QT*>(P.qkv);
   const int head = kvh * P.G + warp;               // this warp's query head
   const int kcol = (P.H + kvh) * HD, vcol = (P.H + P.K + kvh) * HD;
-
-  // ---- Q fragments (A operand, rows = query tokens g and g + 8)
-  uint32_t qa[KS][4];
-  {
-    const int i0 = q0 + g, i1 = q0 + g + 8;
-    const QT* r0 = base + (int64_t)(row0 + (i0 < len ? i0 : len - 1)) * P.ld + head * HD;
-    const QT* r1 = base + (int64_t)(row0 + (i1 < len ? i1 : len - 1)) * P.ld + head * HD;
-#pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-      qa[ks][0] = *reinterpret_cast<const uint32_t*>(r0 + 16 * ks + 2 * tg);
-      qa[ks][1] = *reinterpret_cast<const uint32_t*>(r1 + 16 * ks + 2 * tg);
-      qa[ks][2] = *reinterpret_cast<const uint32_t*>(r0 + 16 * ks + 8 + 2 * tg);
-      qa[ks][3] = *reinterpret_cast<const uint32_t*>(r1 + 16 * ks + 8 + 2 * tg);
-    }
-  }
 
   // ---- key range of the tile: causal (+ window) over the same sequence
   const int q_last = (q0 + PF_QT - 1 < len ? q0 + PF_QT - 1 : len - 1);
@@ -164,6 +152,27 @@ __global__ void __launch_bounds__(512) prefill_attn_kernel(const __grid_constant
   float m_run[2] = {-INFINITY, -INFINITY}, l_run[2] = {0.f, 0.f};
 
   load_tile(t_first, 0);
+  // ---- Q fragments (A operand, rows = query tokens g and g + 8)
+  uint32_t qa[KS][4];
+  {
+    const int i0 = q0 + g, i1 = q0 + g + 8;
+    const QT* r0 = base + (int64_t)(row0 + (i0 < len ? i0 : len - 1)) * P.ld + head * HD;
+    const QT* r1 = base + (int64_t)(row0 + (i1 < len ? i1 : len - 1)) * P.ld + head * HD;
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+      qa[ks][0] = *reinterpret_cast<const uint32_t*>(r0 + 16 * ks + 2 * tg);
+      qa[ks][1] = *reinterpret_cast<const uint32_t*>(r1 + 16 * ks + 2 * tg);
+      qa[ks][2] = *reinterpret_cast<const uint32_t*>(r0 + 16 * ks + 8 + 2 * tg);
+      qa[ks][3] = *reinterpret_cast<const uint32_t*>(r1 + 16 * ks + 8 + 2 * tg);
+    }
+  }
+  float gate[2] = {1.f, 1.f};
+  if (P.gate_vals != nullptr)
+#pragma unroll
+    for (int hr = 0; hr < 2; ++hr) {
+      const int qi = q0 + g + 8 * hr;
+      gate[hr] = P.gate_vals[(int64_t)(row0 + (qi < len ? qi : len - 1)) * P.H + head];
+    }
   for (int t = t_first; t <= t_last; ++t) {
     const int s = (t - t_first) & 1;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -269,7 +278,9 @@ __global__ void __launch_bounds__(512) prefill_attn_kernel(const __grid_constant
     }
     const int64_t row = row0 + (live ? qi : len - 1);
     if (P.xsa_alpha != nullptr) {
-      const QT* vr = base + row * P.ld + vcol;
+      // the token's own v lies in the last key tile, which is still in shared memory
+      const QT* vr = reinterpret_cast<const QT*>(pf_smem + (size_t)(((t_last - t_first) & 1) * 2 + 1) * TILEB +
+                                                 (size_t)((live ? qi : len - 1) - t_last * PF_KT) * ROWB);
       float vv[NT_O][2], n2 = 0.f;
 #pragma unroll
       for (int i = 0; i < NT_O; ++i) {
@@ -296,7 +307,7 @@ __global__ void __launch_bounds__(512) prefill_attn_kernel(const __grid_constant
       }
     }
     if (P.gate_vals != nullptr) {
-      const float gt = P.gate_vals[row * P.H + head];
+      const float gt = gate[hr];
 #pragma unroll
       for (int i = 0; i < NT_O; ++i) z[i][0] = rnd<QT>(z[i][0] * gt), z[i][1] = rnd<QT>(z[i][1] * gt);
     }
