@@ -82,9 +82,11 @@ __device__ __forceinline__ float2 block_sum2(float a, float b, float* red_a, flo
 }
 
 constexpr int NUC_LIST = 1024;  // entries of a nucleus search that one warp takes over
+constexpr int NUC_WALK = 16;    // entries its last pass may move the cut by before the row is bisected instead
 
+// (four blocks a multiprocessor hold 512 rows at once and leave the registers that the loops below want)
 template <typename T>
-__global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const __grid_constant__ SampleParams P) {
+__global__ void __launch_bounds__(SAMPLE_THREADS, 4) sample_kernel(const __grid_constant__ SampleParams P) {
   extern __shared__ float e_sm[];  // V + V/CH floats: chunk t of CH values starts at t * (CH + 1) (bank skew)
   __shared__ float red[SAMPLE_THREADS / 32];
   __shared__ float red_v[SAMPLE_THREADS / 32];
@@ -373,15 +375,19 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const __grid_con
     mine = chunk_sum(cut);
     S = block_sum(mine, red, tid);
   }
-  // ---- nucleus: smallest cut whose strictly-larger mass (inside the top-k set) is below top_p * S
-  if (P.top_p < 1.0f) {
+  // ---- nucleus: smallest cut whose strictly-larger mass (inside the top-k set) is below top_p * S.  A row without mass
+  //      (all NaN, or a precapped one with +inf in it) has no nucleus: nothing is cut and the last index comes out.
+  if (P.top_p < 1.0f && S > 0.f) {
     // Bisection over the bit patterns of e.  A pass over the whole row costs 1.2 us and there are some 30 halvings, so the
     // row is scanned only while more than NUC_LIST entries lie between the bounds; those few then go to a list that one
     // warp finishes on its own.  The lower bound to start from: entries of at most half of (1 - top_p) S / V cannot carry
     // the mass that may be left out.  The list's sums are rounded in another order than the row's: one more pass checks the
-    // result with those, and where it does not hold (the limit falls on the edge of an entry) the next entry is the cut.
+    // result with those, and where it does not hold (the limit falls on the edge of an entry) the next entry is the cut, or the
+    // one after that: sums that differ by some 1e-6 S are a step or two where a row has a tail worth cutting.  A tail of
+    // entries far below that would be walked through entry by entry; after NUC_WALK of them the row is bisected with its own
+    // sums, which ends after 30 halvings whatever the row holds and finds the same cut.
     // 43 -> 24 us at 37 rows of a sharp policy, 35 of normal logits, 110 -> 49 and 81 at 512 (V = 16384).
-    const float lim = P.top_p * S, cut_k = cut;
+    const float lim = fmaxf(P.top_p * S, __uint_as_float(1u)), cut_k = cut;  // (above 0 also where the product is not)
     uint32_t lo = P.top_p < 0.999f ? __float_as_uint(0.5f * (1.0f - P.top_p) * S / (float)V) : 0u;
     uint32_t hi = 0x3f800001u;  // mass_above(hi) = 0 < lim always (e <= 1)
     auto between = [&](float e, uint32_t l, uint32_t h) {
@@ -444,7 +450,9 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const __grid_con
       }
       __syncthreads();
       hi = s_hi;
-      for (;;) {
+      int left = NUC_WALK;
+#pragma unroll 1
+      for (; left > 0; --left) {
         const float ch = __uint_as_float(hi), cl = __uint_as_float(hi - 1u);
         float s1 = 0.f;
         s = 0.f;
@@ -470,6 +478,22 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const __grid_con
         for (int w = 0; w < SAMPLE_THREADS / 32; ++w) next = up ? fminf(next, red[w]) : fmaxf(next, red[w]);
         __syncthreads();
         hi = __float_as_uint(next);
+      }
+      if (left == 0) {
+        lo = 0u, hi = 0x3f800001u;
+#pragma unroll 1
+        while (hi - lo > 1u) {
+          const uint32_t mid = lo + (hi - lo) / 2u;
+          const float cm = __uint_as_float(mid);
+          s = 0.f;
+#pragma unroll 8
+          for (int j = 0; j < CH; ++j) {
+            const float e = chunk[j];
+            s += (e > cm && e >= cut_k) ? e : 0.f;
+          }
+          if (block_sum(s, red, tid) < lim) hi = mid;
+          else lo = mid;
+        }
       }
     }
     cut = fmaxf(__uint_as_float(hi), cut_k);
