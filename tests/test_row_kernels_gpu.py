@@ -14,12 +14,13 @@ def _pieces(n, cut):
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
-@pytest.mark.parametrize("n,d,f", [(768, 640, 1664), (769, 64, 128), (1003, 1032, 4096)])
+@pytest.mark.parametrize("n,d,f", [(768, 640, 1664), (769, 64, 128), (1003, 1032, 4096),
+                                   (800, 320, 8), (771, 2056, 1800)])
 def test_swiglu_of_many_rows(dtype, n, d, f):
     from ultraviolet_b200 import _lib
     from ultraviolet_b200.kernels._util import DTYPE_CODE, stream_ptr
     g = torch.Generator(device="cuda").manual_seed(n)
-    gu = torch.randn(n, 2 * f, device="cuda", generator=g).to(dtype)
+    gu = torch.randn(n, 2 * f, device="cuda", generator=g).to(dtype) * 4
     h = (torch.randn(n, d, device="cuda", generator=g) * 3).to(dtype)
     got, want = (torch.zeros(n, f, device="cuda", dtype=dtype) for _ in range(2))
     for out, cut in ((got, n), (want, 256)):
@@ -31,7 +32,23 @@ def test_swiglu_of_many_rows(dtype, n, d, f):
     ref = torch.nn.functional.silu(x[:, :f]) * x[:, f:]
     tol = 2e-2 if dtype == torch.bfloat16 else 3e-3
     assert torch.allclose(got.float(), ref, rtol=tol, atol=tol * ref.abs().max().item() * 1e-2)
-    assert (got != want).float().mean() < 1e-3       # (norm factors summed in another order: rare last-bit differences)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_swiglu_of_every_value(dtype):
+    """silu of all 65,536 bit patterns: the quotient that many rows take rounds as the one that few rows take."""
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.kernels._util import DTYPE_CODE, stream_ptr
+    n, d, f = 1024, 64, 1024
+    g = torch.arange(n * f, device="cuda").remainder(1 << 16).to(torch.int16).view(dtype).view(n, f)
+    gu, h = torch.cat([g, torch.ones_like(g)], 1), torch.ones(n, d, device="cuda", dtype=dtype)
+    out = [torch.zeros(n, f, device="cuda", dtype=dtype) for _ in range(2)]
+    for o, cut in zip(out, (n, 256)):
+        for a, b in _pieces(n, cut):
+            _lib.check(_lib.lib().uv_swiglu_rs(gu[a:b].data_ptr(), h[a:b].data_ptr(), DTYPE_CODE[dtype], d, f,
+                                               o[a:b].data_ptr(), b - a, stream_ptr(gu.device)), "uv_swiglu_rs")
+    assert torch.equal(out[0].view(torch.int16), out[1].view(torch.int16))
 
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
