@@ -54,7 +54,9 @@ def test_swiglu_of_every_value(dtype):
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("n,H,K,hd,d,pairs,gate,ve,ring", [
     (768, 8, 1, 64, 640, 16, 128, 12, True), (1001, 8, 1, 64, 640, 0, 128, 0, False), (770, 4, 2, 64, 64, 16, 16, 4, True),
-    (800, 3, 1, 128, 1040, 32, 0, 5, False), (900, 6, 2, 32, 192, 8, 24, 12, True)])
+    (800, 3, 1, 128, 1040, 32, 0, 5, False), (900, 6, 2, 32, 192, 8, 24, 12, True),
+    (800, 3, 1, 128, 1000, 64, 0, 128, False), (777, 5, 1, 16, 96, 8, 18, 3, True), (780, 11, 3, 64, 1024, 32, 100, 37, True),
+    (769, 9, 1, 128, 520, 32, 127, 0, True), (768, 1, 1, 32, 8, 16, 8, 1, False)])
 def test_qkv_post_of_many_rows(dtype, n, H, K, hd, d, pairs, gate, ve, ring):
     from ultraviolet_b200 import _lib
     from ultraviolet_b200.kernels._util import DTYPE_CODE, stream_ptr
@@ -96,10 +98,5 @@ def test_qkv_post_of_many_rows(dtype, n, H, K, hd, d, pairs, gate, ve, ring):
         res.append((qkv, gates, kc, vc, ks, vs, oob))
     (q1, g1, *c1, o1), (q2, g2, *c2, o2) = res
     assert int(o1) == int(o2) == (0 if ring else 2 * K)
-    ulp = 2.0 ** -7 if dtype == torch.bfloat16 else 2.0 ** -10
-    assert torch.allclose(q1.float(), q2.float(), rtol=2 * ulp, atol=2 * ulp) and (q1 != q2).float().mean() < 5e-3
-    assert torch.allclose(g1, g2, rtol=2 * ulp, atol=2 * ulp)
-    for a, b in zip(c1[:2], c2[:2]):
-        assert (a.int() - b.int()).abs().max() <= 1 and (a != b).float().mean() < 1e-2
-    for a, b in zip(c1[2:], c2[2:]):
-        assert torch.equal(a == 0, b == 0) and torch.allclose(a.float(), b.float(), rtol=2 * ulp, atol=0)
+    for a, b in zip((q1, g1, *c1), (q2, g2, *c2)):
+        assert torch.equal(a, b)

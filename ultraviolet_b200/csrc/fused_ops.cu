@@ -457,23 +457,55 @@ __global__ void __launch_bounds__(W * 32) qkv_post_kernel(const __grid_constant_
 // from registers that then feed the gates -- and a head slot is a group of HD / 8 lanes with 16 bytes each, so a row of
 // ten 64-wide slots is three passes.  The kernel above spends a warp on every slot and gate, eighteen a row, each with
 // its own chain of loads: right when rows are few, three times the instructions and 2-byte-a-lane traffic when they are
-// not.  20,500 rows: 136 us -> 43 us (78 MB: 12 us at the measured copy rate).
+// not.  20,500 rows: 136 us -> 41 us (78 MB: 12 us at the measured copy rate).
+// The results are those of the kernel above bit for bit (a row's bits must not depend on how many rows came with it): every
+// sum adds the same partial sums in the same order, which takes a butterfly for each of them; lanes that would hold copies
+// of several such sums keep one each instead.  COOP: as the cooperative form of that kernel sums a row's squares, one sum
+// for 256 elements, else one for the row.
 constexpr int QPR_WARPS = 8;
 constexpr int QPR_ROWS = 768;
 constexpr int QPR_GCH = 128;   // channels a gate may read
 
-template <typename T, int HD>
+// N sums over the lanes of a group of LG, each as the butterfly of xor LG/2, ..., 1 adds it, left where the index's high bits
+// are the lane's: v[i] of lane l is sum number (l / (LG / min(LG, N))) * (N / min(LG, N)) + i.
+template <int LG, int N> __device__ __forceinline__ void group_sums(float (&v)[N], int lane) {
+  int n = N;
+#pragma unroll
+  for (int o = LG / 2; o > 0; o >>= 1) {
+    if (n > 1) {
+      n >>= 1;
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < N / 2; ++i)
+        if (i < n) {
+          const float send = up ? v[i] : v[i + n];
+          v[i] = (up ? v[i + n] : v[i]) + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  }
+}
+
+template <typename T, int HD, bool COOP>
 __global__ void __launch_bounds__(QPR_WARPS * 32) qkv_post_rows_kernel(const __grid_constant__ QkvPostParams P) {
   constexpr int LG = HD / 8, NG = 32 / LG;              // lanes a slot, slots a pass
+  constexpr int E = HD >= 32 ? HD / 32 : 1, NP = 8 / E; // elements of a slot that the kernel above has in a lane
   extern __shared__ __align__(16) unsigned char qpr_smem[];
-  T* const gw = reinterpret_cast<T*>(qpr_smem);         // (H, gate_ch) then (K, ve_ch)
-  T* const vw = gw + (P.gate_out ? P.H * P.gate_ch : 0);
+  // (H, 32, 4) then (K, 32, 4): channels lane, lane + 32, lane + 64, lane + 96 of a gate side by side, zeros past its last
+  T* const gw = reinterpret_cast<T*>(qpr_smem);
+  T* const vw = gw + (P.gate_out ? P.H * QPR_GCH : 0);
   const int lane = threadIdx.x & 31, grp = lane / LG, gl = lane % LG;
   const int slots = P.H + 2 * P.K;
-  if (P.gate_out)
-    for (int i = threadIdx.x; i < P.H * P.gate_ch; i += QPR_WARPS * 32) gw[i] = static_cast<const T*>(P.gate_w)[i];
-  if (P.ve_gate)
-    for (int i = threadIdx.x; i < P.K * P.ve_ch; i += QPR_WARPS * 32) vw[i] = static_cast<const T*>(P.ve_gate)[i];
+  auto stage = [&](T* to, const void* from, int n, int channels) {
+    for (int i = threadIdx.x; i < n * QPR_GCH; i += QPR_WARPS * 32) {
+      const int c = ((i >> 2) & 31) + 32 * (i & 3);
+      to[i] = c < channels ? static_cast<const T*>(from)[(i / QPR_GCH) * channels + c] : from_f32<T>(0.f);
+    }
+  };
+  if (P.gate_out) stage(gw, P.gate_w, P.H, P.gate_ch);
+  if (P.ve_gate) stage(vw, P.ve_gate, P.K, P.ve_ch);
+  const int channels = max(P.gate_out ? P.gate_ch : 0, P.ve_gate ? P.ve_ch : 0);
   pdl_wait();
   pdl_trigger();
   __syncthreads();
@@ -496,10 +528,17 @@ __global__ void __launch_bounds__(QPR_WARPS * 32) qkv_post_rows_kernel(const __g
       v[k] = r.x, v[k + 1] = r.y;
     }
   };
-  auto group_sum = [](float v) {
-#pragma unroll
-    for (int o = LG / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+  // this lane's share of one gate's product with the normalised channels, in the order of head_gate
+  auto gate_dot = [](const float (&xs)[4], const T* w) {
+    const uint2 u = *reinterpret_cast<const uint2*>(w);
+    const typename Vec2<T>::type* h = reinterpret_cast<const typename Vec2<T>::type*>(&u);
+    float acc = 0.f;
+    acc += xs[0] * to_f32<T>(h[0].x), acc += xs[1] * to_f32<T>(h[0].y);
+    acc += xs[2] * to_f32<T>(h[1].x), acc += xs[3] * to_f32<T>(h[1].y);
+    return acc;
+  };
+  auto gate_of = [](float dot) {
+    return rnd<T>(2.0f * rnd<T>(1.0f / (1.0f + __expf(-rnd<T>(dot)))));
   };
   auto group_max = [](float v) {
 #pragma unroll
@@ -515,46 +554,40 @@ __global__ void __launch_bounds__(QPR_WARPS * 32) qkv_post_rows_kernel(const __g
       const int i = 8 * lane + 256 * j;
       xu[j] = i < P.d ? *reinterpret_cast<const uint4*>(xr + i) : make_uint4(0u, 0u, 0u, 0u);
     }
+    float xs[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) xs[j] = lane + 32 * j < channels ? to_f32<T>(xr[lane + 32 * j]) : 0.f;
     uint4 raw = grp < slots ? *reinterpret_cast<const uint4*>(qr + grp * HD + 8 * gl) : make_uint4(0u, 0u, 0u, 0u);
     const QkvSlot dest = qkv_post_slot(P, b);
     const float* cs = P.inv_freq ? P.rope_cs + (int64_t)b * 2 * P.n_pairs : nullptr;
-    float ss = 0.f, x[8];
+    float x[8], part[4] = {0.f, 0.f, 0.f, 0.f}, ss;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       unpack(xu[j], x);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) ss += x[k] * x[k];
+      for (int k = 0; k < 8; ++k) part[COOP ? j : 0] += x[k] * x[k];
     }
-    for (int i = 8 * lane + 1024; i < P.d; i += 256) {  // rows wider than 1024 elements
-      unpack(*reinterpret_cast<const uint4*>(xr + i), x);
+    if constexpr (COOP) {
+      group_sums<32, 4>(part, lane);
+      ss = __shfl_sync(0xffffffffu, part[0], 0);
 #pragma unroll
-      for (int k = 0; k < 8; ++k) ss += x[k] * x[k];
+      for (int j = 1; j < 4; ++j) ss += __shfl_sync(0xffffffffu, part[0], 8 * j);
+    } else {
+      ss = warp_sum(part[0]);
     }
-    const float rs = rsqrtf(warp_sum(ss) / (float)P.d + RMS_EPS);
-    // ---- gates: the row's first 128 channels, normalised, 8 in each lane of both half-warps
-    float xc[8];
-    {
-      const uint4 u = make_uint4(__shfl_sync(0xffffffffu, xu[0].x, lane & 15), __shfl_sync(0xffffffffu, xu[0].y, lane & 15),
-                                 __shfl_sync(0xffffffffu, xu[0].z, lane & 15), __shfl_sync(0xffffffffu, xu[0].w, lane & 15));
-      unpack(u, xc);
-      scale(xc, rs);
-    }
+    const float rs = rsqrtf(ss / (float)P.d + RMS_EPS);
+    // ---- head gates, eight at a time
+#pragma unroll
+    for (int j = 0; j < 4; ++j) xs[j] = rnd<T>(xs[j] * rs);
     if (P.gate_out) {
-      const int c = 8 * (lane & 15);
-      for (int h0 = 0; h0 < P.H; h0 += 2) {             // a head per half-warp
-        const int h = h0 + (lane >> 4);
-        float acc = 0.f;
-        if (h < P.H && c < P.gate_ch) {
-          float w[8];
-          unpack(*reinterpret_cast<const uint4*>(gw + h * P.gate_ch + c), w);
+      for (int h0 = 0; h0 < P.H; h0 += 8) {
+        float dot[8];
 #pragma unroll
-          for (int k = 0; k < 8; ++k) acc += xc[k] * w[k];
-        }
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        acc = rnd<T>(acc);
-        const float g = rnd<T>(2.0f * rnd<T>(__fdividef(1.0f, 1.0f + __expf(-acc))));
-        if (h < P.H && (lane & 15) == 0) P.gate_out[(int64_t)b * P.H + h] = g;
+        for (int i = 0; i < 8; ++i) dot[i] = h0 + i < P.H ? gate_dot(xs, gw + ((h0 + i) * 32 + lane) * 4) : 0.f;
+        group_sums<32, 8>(dot, lane);
+        const int h = h0 + (lane >> 2);
+        const float g = gate_of(dot[0]);
+        if (h < P.H && (lane & 3) == 0) P.gate_out[(int64_t)b * P.H + h] = g;
       }
     }
     // ---- head slots, NG at a time
@@ -566,10 +599,24 @@ __global__ void __launch_bounds__(QPR_WARPS * 32) qkv_post_rows_kernel(const __g
         raw = hs + NG < slots ? *reinterpret_cast<const uint4*>(qr + (hs + NG) * HD + 8 * gl) : make_uint4(0u, 0u, 0u, 0u);
       unpack(cur, x);
       scale(x, rs);
-      ss = 0.f;
+      float sq[NP];
 #pragma unroll
-      for (int k = 0; k < 8; ++k) ss += x[k] * x[k];
-      const float inv = rsqrtf(group_sum(ss) / (float)HD + RMS_EPS);
+      for (int i = 0; i < NP; ++i) {
+        sq[i] = 0.f;
+#pragma unroll
+        for (int k = 0; k < E; ++k) sq[i] += x[i * E + k] * x[i * E + k];
+      }
+      group_sums<LG, NP>(sq, lane);
+      constexpr int LEFT = NP > LG ? NP / LG : 1;       // sums that stayed in a lane, then added in the butterfly's order
+#pragma unroll
+      for (int o = LG / 2, m = NP; o > 0 && m > 1; o >>= 1, m >>= 1)
+#pragma unroll
+        for (int i = 0; i < LEFT; ++i) sq[i] += __shfl_xor_sync(0xffffffffu, sq[i], o);
+#pragma unroll
+      for (int m = LEFT / 2; m > 0; m >>= 1)
+#pragma unroll
+        for (int i = 0; i < m; ++i) sq[i] += sq[i + m];
+      const float inv = rsqrtf(sq[0] / (float)HD + RMS_EPS);
       if (!isv) scale(x, inv);
       if (cs != nullptr) {                              // dim j < n_pairs turns with dim j + n_pairs
         const int np8 = P.n_pairs / 8;
@@ -589,18 +636,13 @@ __global__ void __launch_bounds__(QPR_WARPS * 32) qkv_post_rows_kernel(const __g
       }
       if (P.ve_gate != nullptr && s0 + NG > P.H + P.K) {  // some slot of this pass is a value head (warp-uniform)
         const int kh = isv && live ? hs - P.H - P.K : 0;
-        float acc = 0.f;                                // channels 8 i .. 8 i + 7 sit in lane i
+        float acc = 0.f;
         for (int k0 = 0; k0 < P.K; ++k0) {
-          float p = 0.f;
-#pragma unroll
-          for (int k = 0; k < 8; ++k)
-            if (lane < 16 && 8 * lane + k < P.ve_ch) p += xc[k] * to_f32<T>(vw[k0 * P.ve_ch + 8 * lane + k]);
-          p = warp_sum(p);
+          const float p = warp_sum(gate_dot(xs, vw + (k0 * 32 + lane) * 4));
           if (k0 == kh) acc = p;
         }
         if (isv && live) {
-          acc = rnd<T>(acc);
-          const float g = rnd<T>(2.0f * rnd<T>(__fdividef(1.0f, 1.0f + __expf(-acc))));
+          const float g = gate_of(acc);
           int64_t t = P.tok[b];
           if (t < 0 || t >= P.vocab) t = 0;
           float ve[8];
@@ -653,32 +695,38 @@ template <typename T>
 static int launch_qkv_post(const QkvPostParams& P, int hd, cudaStream_t st) {
   const int per_row = P.H + 2 * P.K + (P.gate_out ? P.H : 0);
   const int64_t items = (int64_t)P.B * per_row;
-  // many rows: a warp a row.  Below QPR_ROWS rows a row's own chain is what counts, and a warp for every slot shortens it
-  // (256 rows: 4.2 us against 7.0; 768: 7.7 against 7.3; 4096: 12.9 with this one).
-  const bool rows_ok = P.B >= QPR_ROWS && P.xn_raw && (!P.gate_out || (P.gate_ch <= QPR_GCH && P.gate_ch % 8 == 0)) &&
-                       (!P.ve_gate || P.ve_ch <= QPR_GCH) && aligned16(P.qkv) &&
-                       (!P.ve_gate || aligned16(P.value_embed)) &&
-                       (!P.k_cache || (((uintptr_t)P.k_cache | (uintptr_t)P.v_cache) & 7) == 0) &&
-                       (!P.inv_freq || (P.rope_cs && (P.n_pairs == 8 || P.n_pairs == 16 || P.n_pairs == 32 || P.n_pairs == 64)));
-  if (rows_ok) {
-    const size_t smem = ((P.gate_out ? (size_t)P.H * P.gate_ch : 0) + (P.ve_gate ? (size_t)P.K * P.ve_ch : 0)) * sizeof(T);
-    const int64_t ctas = ((int64_t)P.B + QPR_WARPS - 1) / QPR_WARPS;
-    const unsigned grid = (unsigned)(ctas < 148 * 6 ? ctas : 148 * 6);
-    switch (hd) {
-      case 16: launch_pdl(qkv_post_rows_kernel<T, 16>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
-      case 32: launch_pdl(qkv_post_rows_kernel<T, 32>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
-      case 64: launch_pdl(qkv_post_rows_kernel<T, 64>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
-      case 128: launch_pdl(qkv_post_rows_kernel<T, 128>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P); break;
-      default: return UV_ERR_SHAPE;
-    }
-    return check_launch();
-  }
   // cooperative row reduction when the launch defers the norm and a row's items fill whole CTAs of 6 or 4 warps
   static const bool coop_on = [] {
     const char* v = getenv("UVDECODE_QKV_POST_COOP");
     return !(v && v[0] == '0');
   }();
   const int coop = (P.xn_raw && coop_on) ? (per_row % 6 == 0 ? 6 : (per_row % 4 == 0 ? 4 : 0)) : 0;
+  // many rows: a warp a row.  Below QPR_ROWS rows a row's own chain is what counts, and a warp for every slot shortens it
+  // (256 rows: 4.2 us against 7.0; 768: 7.7 against 7.3; 4096: 12.9 with this one).
+  const bool rows_ok = P.B >= QPR_ROWS && P.xn_raw && P.d <= 1024 && (!P.gate_out || P.gate_ch <= QPR_GCH) &&
+                       (!P.ve_gate || P.ve_ch <= QPR_GCH) && aligned16(P.qkv) &&
+                       (!P.ve_gate || aligned16(P.value_embed)) &&
+                       (!P.k_cache || (((uintptr_t)P.k_cache | (uintptr_t)P.v_cache) & 7) == 0) &&
+                       (!P.inv_freq || (P.rope_cs && (P.n_pairs == 8 || P.n_pairs == 16 || P.n_pairs == 32 || P.n_pairs == 64)));
+  if (rows_ok) {
+    const size_t smem = (size_t)((P.gate_out ? P.H : 0) + (P.ve_gate ? P.K : 0)) * QPR_GCH * sizeof(T);
+    const int64_t ctas = ((int64_t)P.B + QPR_WARPS - 1) / QPR_WARPS;
+    const unsigned grid = (unsigned)(ctas < 148 * 6 ? ctas : 148 * 6);
+#define UV_QKV_POST_ROWS(HD_)                                                                                             \
+  case HD_:                                                                                                               \
+    if (coop) launch_pdl(qkv_post_rows_kernel<T, HD_, true>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P);              \
+    else launch_pdl(qkv_post_rows_kernel<T, HD_, false>, dim3(grid), dim3(QPR_WARPS * 32), smem, st, P);                  \
+    break;
+    switch (hd) {
+      UV_QKV_POST_ROWS(16)
+      UV_QKV_POST_ROWS(32)
+      UV_QKV_POST_ROWS(64)
+      UV_QKV_POST_ROWS(128)
+      default: return UV_ERR_SHAPE;
+    }
+#undef UV_QKV_POST_ROWS
+    return check_launch();
+  }
   const int wpc = coop ? coop : 4;
   const unsigned grid = (unsigned)((items + wpc - 1) / wpc);
   // with the step's RoPE table the kernel carries no cosf / sinf code at all
