@@ -324,7 +324,8 @@ class DecodeEngine:
     # ------------------------------------------------------------------------------------------------ one step
     def trunk(self, tok: Tensor, st, pos: Tensor, starts: Tensor, g_len: int | None = None,
               num_splits: dict | None = None, row_map: Tensor | None = None, skip_attn: bool = False,
-              packed: dict | None = None, scratch_tag: str = "", shared_rows: bool = False) -> Tensor:
+              packed: dict | None = None, scratch_tag: str = "", shared_rows: bool = False,
+              one_launch: bool = True) -> Tensor:
         """One token for every batch entry: writes K/V at `pos` and returns the final normed hidden (B, d) (a view
         of engine scratch, overwritten by the next call).  pos/starts are batch-indexed (B,) int64; row_map
         optionally maps batch entries to cache rows.
@@ -336,7 +337,10 @@ class DecodeEngine:
         only the newest positions of each prompt.
 
         shared_rows: several entries of this call may be tokens of one sequence and read each other's keys (prefill
-        lanes): every layer's append then has to finish before its attention starts."""
+        lanes): every layer's append then has to finish before its attention starts.
+
+        one_launch=False: one launch per operation also where uv_decode_step would take the batch (the two round the
+        same activations from sums in different orders)."""
         cfg, lib, dt = self.cfg, _lib.lib(), DTYPE_CODE[self.dtype]
         B = tok.size(0)
         s = self.scratch(B, scratch_tag)
@@ -348,7 +352,7 @@ class DecodeEngine:
         fused = self.fused_gemm and packed is None
         qkv_in_attn = self.qkv_in_attn and packed is None
         fold = self.fold
-        if self.one_launch and packed is None and not skip_attn and not shared_rows and not ns:
+        if self.one_launch and one_launch and packed is None and not skip_attn and not shared_rows and not ns:
             with torch.cuda.device(self.device):
                 a = self._step_args(tok, st, pos, starts, rm, s)
                 if lib.uv_decode_step_supported(C.byref(a)):
