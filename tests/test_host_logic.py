@@ -140,3 +140,19 @@ def test_bench_workload_definitions_are_deterministic_and_match_their_configurat
     assert bench.attn_bytes(pos, starts, 256, S=256, ring=True) == (10 + 256 + 3) * 132 + 2 * 3 * 8 * 64 * 2
     cfg = bench.workload_config(20)
     assert cfg == bench.workload_config(20) and "workload" in cfg
+
+
+def test_default_matmul_sees_every_switch():
+    """Native code calls cuBLAS itself only while torch's matrix products are the plain call."""
+    import torch
+    from ultraviolet_b200.engine import default_matmul
+    mm = torch.backends.cuda.matmul
+    assert default_matmul()
+    for name in ("allow_fp16_reduced_precision_reduction", "allow_bf16_reduced_precision_reduction", "allow_fp16_accumulation"):
+        before = getattr(mm, name)
+        setattr(mm, name, not before)
+        try:
+            assert not default_matmul()
+        finally:
+            setattr(mm, name, before)
+    assert default_matmul()

@@ -78,3 +78,43 @@ def test_softcap(shape, dtype):
     _lib.check(_lib.lib().uv_softcap(x.data_ptr(), DTYPE_CODE[dtype], x.numel(), 23.0, 5.0, 7.5, out.data_ptr(),
                                      stream_ptr(x.device)), "uv_softcap")
     assert torch.allclose(out, 23.0 * torch.sigmoid((x.float() + 5.0) / 7.5), rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("switch", [None, "allow_fp16_reduced_precision_reduction", "allow_bf16_reduced_precision_reduction",
+                                    "allow_fp16_accumulation", "library"])
+def test_prefill_follows_the_switches_of_matmul(dtype, switch, monkeypatch):
+    """The native prompt pass gives the bits of the one that calls torch.mm, whatever torch's matrix products are set to."""
+    from ultraviolet_b200.engine import DecodeEngine
+    from ultraviolet_b200.model import MathLM, make_config
+    torch.manual_seed(5)
+    with torch.device("cuda"):
+        m = MathLM(make_config("uv-50m-alpha", vocab_size=500, n_layers=3, global_every=2))
+    with torch.no_grad():
+        for b in m.blocks:
+            b.attn.wo.normal_(std=0.02), b.mlp.w_down.normal_(std=0.02)
+    m = m.to(dtype).fuse_for_inference(dtype)
+    lens, T = torch.tensor([300, 1, 17, 290, 260]), 300
+    idx = torch.randint(1, 500, (5, T), device="cuda")
+    starts = (T - lens).cuda()
+    mm = torch.backends.cuda.matmul
+    before = mm.allow_fp16_accumulation if switch == "allow_fp16_accumulation" else True
+    lib = torch.backends.cuda.preferred_blas_library()
+    try:
+        if switch == "library":
+            torch.backends.cuda.preferred_blas_library("cublaslt")
+        elif switch:
+            setattr(mm, switch, not before)
+        assert (m.engine.prefill_trunk() is None) == bool(switch)
+        res = []
+        for native in (True, False):
+            if not native:
+                monkeypatch.setattr(DecodeEngine, "prefill_trunk", lambda self: None)
+            st = m.new_state(5, T + 8)
+            res.append((m.prefill(idx, starts, st), *st.k, *st.v, *st.k_scale, *st.v_scale))
+        for a, b in zip(*res):
+            assert torch.equal(a, b)
+    finally:
+        torch.backends.cuda.preferred_blas_library(lib)
+        if switch and switch != "library":
+            setattr(mm, switch, before)

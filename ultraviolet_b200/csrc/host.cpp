@@ -176,8 +176,8 @@ std::optional<std::pair<Tensor, Tensor>> fused_sample(const Tensor& x, const Ten
 }
 
 // c = x . w^T (accumulate: c += x . w^T) for contiguous row-major x (M, K), w (N, K), c (M, N): the cuBLAS call that torch.mm
-// makes (torch's handle, workspace and stream; fp32 accumulation), without the operator dispatch in front of it, which
-// costs more than the launch
+// makes (torch's handle, workspace and stream; fp32 accumulation) while its switches are at their defaults
+// (engine.py: default_matmul), without the operator dispatch in front of it, which costs more than the launch
 void gemm(const Tensor& x, const Tensor& w, Tensor& c, bool accumulate = false) {
   const int M = (int)x.size(0), K = (int)x.size(1), N = (int)w.size(0);
   if (M == 0) return;

@@ -32,6 +32,15 @@ def _align(n: int, a: int = 128) -> int:
     return (n + a - 1) // a * a
 
 
+def default_matmul() -> bool:
+    """torch's matrix products run as a plain cuBLAS call with fp32 accumulation: no switch of the program asks for other
+    reductions, another library or tuned kernels.  Native code that calls cuBLAS itself does so only then."""
+    mm = torch.backends.cuda.matmul
+    return (mm.allow_fp16_reduced_precision_reduction is True and mm.allow_bf16_reduced_precision_reduction is True
+            and not mm.allow_fp16_accumulation and not torch.cuda.tunable.is_enabled()
+            and torch.backends.cuda.preferred_blas_library() == torch._C._BlasBackend.Cublas)
+
+
 class DecodeEngine:
     def __init__(self, cfg: MathConfig, dtype: torch.dtype, device):
         cfg.check_decode_supported()
@@ -631,8 +640,9 @@ class DecodeEngine:
         return out
 
     def prefill_trunk(self):
-        """The native host loop of a packed prompt pass (None: this engine runs its trunk another way)."""
-        if not self.fold or self.sw_qkv != "0" or not self.rope_table:
+        """The native host loop of a packed prompt pass (None: this engine runs its trunk another way, or torch's matrix
+        products are not the library call that the loop makes)."""
+        if not self.fold or self.sw_qkv != "0" or not self.rope_table or not default_matmul():
             return None
         if self._prefill_trunk is None:
             cfg, w, L = self.cfg, self.w, range(self.cfg.n_layers)
