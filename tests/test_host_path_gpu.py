@@ -118,3 +118,30 @@ def test_prefill_follows_the_switches_of_matmul(dtype, switch, monkeypatch):
         torch.backends.cuda.preferred_blas_library(lib)
         if switch and switch != "library":
             setattr(mm, switch, before)
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_prefill_keeps_no_buffers_per_length(native, monkeypatch):
+    """Prompts of many lengths one after the other: what a pass allocated is given back (native pass) or shared by the lengths of a
+    bucket (the pass through ``trunk``), and its count of skipped cache writes is read with the other failure words."""
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.engine import DecodeEngine
+    from ultraviolet_b200.model import MathLM, make_config
+    torch.manual_seed(6)
+    with torch.device("cuda"):
+        m = MathLM(make_config("uv-50m-alpha", vocab_size=500, n_layers=2)).bfloat16().fuse_for_inference()
+    if not native:
+        monkeypatch.setattr(DecodeEngine, "prefill_trunk", lambda self: None)
+    eng, st = m.engine, m.new_state(1, 2200)
+    used = []
+    for T in (2150, 2049, *range(1, 130, 3), 1000, 2048):
+        m.prefill(torch.ones(1, T, dtype=torch.long, device="cuda"), torch.zeros(1, dtype=torch.long, device="cuda"), st)
+        used.append(torch.cuda.memory_allocated())
+    if native:
+        assert not eng._scratch and max(used[1:]) == min(used[1:])
+        eng.prefill_oob()[0] = 2
+        with pytest.raises(_lib.UvError):
+            eng.check_status(1)
+        assert eng.device_status() == {"attn_status": 0, "kv_oob": 0}
+    else:
+        assert sorted(k[0] for k in eng._scratch) == [64, 128, 1024, 2048, 4096]        # (1 ... 127, 1000, 2048, 2049, 2150)

@@ -178,14 +178,13 @@ std::optional<std::pair<Tensor, Tensor>> fused_sample(const Tensor& x, const Ten
 // c = x . w^T (accumulate: c += x . w^T) for contiguous row-major x (M, K), w (N, K), c (M, N): the cuBLAS call that torch.mm
 // makes (torch's handle, workspace and stream; fp32 accumulation) while its switches are at their defaults
 // (engine.py: default_matmul), without the operator dispatch in front of it, which costs more than the launch
-void gemm(const Tensor& x, const Tensor& w, Tensor& c, bool accumulate = false) {
-  const int M = (int)x.size(0), K = (int)x.size(1), N = (int)w.size(0);
-  if (M == 0) return;
-  const cudaDataType_t type = x.scalar_type() == at::kHalf ? CUDA_R_16F : CUDA_R_16BF;
+void gemm(int M, const void* x, const Tensor& w, void* c, bool accumulate = false) {
+  const int K = (int)w.size(1), N = (int)w.size(0);
+  const cudaDataType_t type = w.scalar_type() == at::kHalf ? CUDA_R_16F : CUDA_R_16BF;
   const float one = 1.0f, beta = accumulate ? 1.0f : 0.0f;
   const cublasStatus_t s = cublasGemmEx(at::cuda::getCurrentCUDABlasHandle(), CUBLAS_OP_T, CUBLAS_OP_N, N, M, K, &one,
-                                        ro(w), type, K, ro(x), type, K, &beta, c.mutable_data_ptr(), type, N,
-                                        CUBLAS_COMPUTE_32F, CUBLAS_GEMM_DEFAULT_TENSOR_OP);
+                                        ro(w), type, K, x, type, K, &beta, c, type, N, CUBLAS_COMPUTE_32F,
+                                        CUBLAS_GEMM_DEFAULT_TENSOR_OP);
   TORCH_CHECK(s == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed with status ", (int)s);
 }
 
@@ -214,17 +213,27 @@ class PrefillTrunk {
     code_ = code_of(embed.scalar_type());
   }
 
-  // x .. act, gate, rope_cs, oob: scratch rows of this pass; k .. vs: the state's layers.  The un-normalised final stream
-  // of the pass is left in x; the normed rows of the prompts' last tokens are returned (zeros for an empty prompt).
-  Tensor run(const Tensor& idx, const Tensor& starts, const Tensor& rows, int64_t M, int64_t max_tiles, Tensor x, Tensor xn,
-             Tensor qkv, Tensor z, Tensor gu, Tensor act, Tensor gate, Tensor rope_cs, Tensor oob,
+  // oob: device word that counts skipped cache writes; k .. vs: the state's layers.  Returns the normed rows of the prompts'
+  // last tokens (zeros for an empty prompt).  M >= 1.
+  Tensor run(const Tensor& idx, const Tensor& starts, const Tensor& rows, int64_t M, int64_t max_tiles, Tensor oob,
              const std::vector<Tensor>& k, const std::vector<Tensor>& v, const std::vector<Tensor>& ks,
              const std::vector<Tensor>& vs) {
     at::AutoDispatchBelowADInplaceOrView below;         // no autograd bookkeeping on the library calls below
-    c10::cuda::CUDAGuard guard(x.device());
+    c10::cuda::CUDAGuard guard(embed_.device());
     void* st = at::cuda::getCurrentCUDAStream().stream();
     const int n = (int)idx.size(0), T = (int)idx.size(1), d = (int)embed_.size(1), m = (int)M;
     const int64_t vocab = embed_.size(0);
+    // The activations of the pass, one block of the allocator's pool that goes back to it at the end: passes come in every
+    // size, so buffers kept per size would add up without bound, and passes on several streams or threads have their own.
+    const int slots = H_ + 2 * K_;
+    const int64_t widths[8] = {2 * d, 2 * d, 2 * slots * hd_, 2 * H_ * hd_, 4 * f_, 2 * f_, 4 * H_, 8 * n_pairs_};
+    int64_t at[9] = {0};
+    for (int b = 0; b < 8; ++b) at[b + 1] = at[b] + (widths[b] * M + 255) / 256 * 256;
+    const Tensor block = at::empty({at[8]}, embed_.options().dtype(at::kByte));
+    char* const base = static_cast<char*>(block.mutable_data_ptr());
+    void *const x = base, *const xn = base + at[1], *const qkv = base + at[2], *const z = base + at[3];
+    void *const gu = base + at[4], *const act = base + at[5];
+    float *const gate = reinterpret_cast<float*>(base + at[6]), *const rope_cs = reinterpret_cast<float*>(base + at[7]);
     // tok, pos, row, last of every packed row and the two prefix sums, in one allocation each
     Tensor packed = at::empty({4, M}, idx.options()), cu = at::empty({2, n + 1}, idx.options().dtype(at::kInt));
     int64_t *tok = packed.mutable_data_ptr<int64_t>(), *pos = tok + M, *row = pos + M, *last = row + M;
@@ -233,38 +242,38 @@ class PrefillTrunk {
                          rows.const_data_ptr<int64_t>(), n, M, cu_p, tile_p, tok, pos, row, last, st),
           "uv_pack_prompts");
     if (n_pairs_ > 0)
-      check(L.embed_norm_rope(tok, ro(embed_), code_, vocab, d, x.mutable_data_ptr(), xn.mutable_data_ptr(), m, pos,
-                              inv_freq_.const_data_ptr<float>(), n_pairs_, rope_cs.mutable_data_ptr<float>(), st),
+      check(L.embed_norm_rope(tok, ro(embed_), code_, vocab, d, x, xn, m, pos, inv_freq_.const_data_ptr<float>(), n_pairs_, rope_cs,
+                              st),
             "uv_embed_norm_rope");
     else
-      check(L.embed_norm(tok, ro(embed_), code_, vocab, d, x.mutable_data_ptr(), xn.mutable_data_ptr(), m, st), "uv_embed_norm");
+      check(L.embed_norm(tok, ro(embed_), code_, vocab, d, x, xn, m, st), "uv_embed_norm");
     for (size_t l = 0; l < layers_.size(); ++l) {
       const LayerFacts& y = layers_[l];
-      gemm(x, y.wqkv, qkv);
+      gemm(m, x, y.wqkv, qkv);
       uv_qkv_args q{};
-      q.qkv = qkv.mutable_data_ptr(), q.xn = ro(x), q.tok = tok, q.pos = pos, q.row_map = row, q.last_pos = last;
+      q.qkv = qkv, q.xn = x, q.tok = tok, q.pos = pos, q.row_map = row, q.last_pos = last;
       q.value_embed = value_embed_ ? ro(*value_embed_) : nullptr, q.ve_gate = y.ve_gate;
-      if (y.rope && n_pairs_ > 0) q.inv_freq = inv_freq_.const_data_ptr<float>(), q.rope_cs = rope_cs.const_data_ptr<float>();
+      if (y.rope && n_pairs_ > 0) q.inv_freq = inv_freq_.const_data_ptr<float>(), q.rope_cs = rope_cs;
       q.k_cache = k[l].mutable_data_ptr<int8_t>(), q.v_cache = v[l].mutable_data_ptr<int8_t>();
       q.k_scale = static_cast<uint16_t*>(ks[l].mutable_data_ptr()), q.v_scale = static_cast<uint16_t*>(vs[l].mutable_data_ptr());
       q.oob_count = oob.mutable_data_ptr<int>(), q.dtype = code_, q.vocab = vocab, q.B = m, q.H = H_, q.K = K_, q.hd = hd_;
       q.d = d, q.S = (int)k[l].size(2), q.S_alloc = (int)(k[l].stride(1) / hd_), q.ring = y.ring, q.ve_ch = ve_ch_;
       q.n_pairs = n_pairs_, q.xn_raw = 1;
-      if (gate_ch_ > 0) q.gate_w = y.attn_gate, q.gate_out = gate.mutable_data_ptr<float>(), q.gate_ch = gate_ch_;
+      if (gate_ch_ > 0) q.gate_w = y.attn_gate, q.gate_out = gate, q.gate_ch = gate_ch_;
       check(L.qkv_post(&q, st), "uv_qkv_post");
       uv_prefill_attn_args p{};
-      p.qkv = ro(qkv), p.dtype = code_, p.ld = qkv.stride(0), p.cu_seqlens = cu_p, p.tile_cu = tile_p, p.n_seq = n;
-      p.max_tiles = (int)max_tiles, p.out = z.mutable_data_ptr(), p.ldo = z.stride(0), p.H = H_, p.K = K_, p.hd = hd_;
+      p.qkv = qkv, p.dtype = code_, p.ld = slots * hd_, p.cu_seqlens = cu_p, p.tile_cu = tile_p, p.n_seq = n;
+      p.max_tiles = (int)max_tiles, p.out = z, p.ldo = H_ * hd_, p.H = H_, p.K = K_, p.hd = hd_;
       p.window = y.window, p.scale = scale_, p.xsa_alpha = y.xsa_alpha, p.xsa_eps = eps_;
-      if (gate_ch_ > 0) p.gate_vals = gate.const_data_ptr<float>();
+      if (gate_ch_ > 0) p.gate_vals = gate;
       check(L.prefill_attn(&p, st), "uv_prefill_attn");
-      gemm(z, y.wo, x, true);
-      gemm(x, y.gu, gu);
-      check(L.swiglu_rs(ro(gu), ro(x), code_, d, f_, act.mutable_data_ptr(), m, st), "uv_swiglu_rs");
-      gemm(act, y.down, x, true);
+      gemm(m, z, y.wo, x, true);
+      gemm(m, x, y.gu, gu);
+      check(L.swiglu_rs(gu, x, code_, d, f_, act, m, st), "uv_swiglu_rs");
+      gemm(m, act, y.down, x, true);
     }
-    Tensor out = at::empty({n, d}, x.options());
-    check(L.gather_norm(ro(x), code_, d, cu_p, n, out.mutable_data_ptr(), st), "uv_gather_norm");
+    Tensor out = at::empty({n, d}, embed_.options());
+    check(L.gather_norm(x, code_, d, cu_p, n, out.mutable_data_ptr(), st), "uv_gather_norm");
     return out;
   }
 

@@ -82,7 +82,7 @@ class DecodeEngine:
         if cfg.rope_pairs:
             self.inv_freq.copy_((1.0 / cfg.rope_base) ** torch.linspace(0, 1, cfg.rope_pairs, dtype=torch.float32))
         self._scratch: dict[int, dict] = {}
-        self._prefill_trunk = None
+        self._prefill_trunk = self._prefill_flags = self._prefill_oob = None
         self._fuse_plan = None      # load_from's launch arguments for the parameter tensors it saw last
         self._fuse_status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.version = 0
@@ -253,11 +253,13 @@ class DecodeEngine:
     BIG_ROWS = 2048  # batches above this (packed prompt prefill) share bucketed buffers instead of one set per size
 
     def scratch(self, B: int, tag: str = "") -> dict:
-        """The buffers of a B-row trunk call.  tag names a second, independent family of buffers for calls that may
-        run beside the untagged ones on another stream (admission passes next to decode steps)."""
-        if B > self.BIG_ROWS:
-            # prefill batches come in every size: one allocation per 4096-row bucket, handed out as [:B] views
-            cap = (B + 4095) // 4096 * 4096
+        """The buffers of a B-row trunk call.  tag names a second, independent family of buffers: "admit" for passes that may
+        run beside the untagged calls on another stream (admission next to decode steps), "prefill" for prompt passes
+        that go through ``trunk``."""
+        if B > self.BIG_ROWS or tag == "prefill":
+            # prompt passes come in every size: one allocation per bucket of 4096 rows, or per power of two from 64 rows
+            # on where that is less, handed out as [:B] views
+            cap = (B + 4095) // 4096 * 4096 if B > self.BIG_ROWS else max(64, 1 << (B - 1).bit_length())
             big = self._scratch.get((cap, tag) if tag else cap) or self.scratch_exact(cap, tag)
             return {k: (v[:B] if isinstance(v, Tensor) and v.dim() >= 1 and v.size(0) == cap and k not in
                         ("flags", "status", "oob") else v) for k, v in big.items()}
@@ -286,14 +288,26 @@ class DecodeEngine:
             self._scratch[key] = s
         return s
 
+    def prefill_oob(self) -> Tensor:
+        """The count of cache writes that native prompt passes skipped (their ``flags`` are those of a scratch set)."""
+        if self._prefill_oob is None:
+            self._prefill_flags = torch.zeros(2, dtype=torch.int32, device=self.device)
+            self._prefill_oob = self._prefill_flags[1:]
+        return self._prefill_oob
+
+    def _flags(self, B: int | None) -> list:
+        sets = [s["flags"] for b, s in self._scratch.items()
+                if B is None or b == B or (isinstance(b, tuple) and b[0] == B)]
+        return sets + ([] if self._prefill_flags is None else [self._prefill_flags])
+
     def device_status(self, B: int | None = None) -> dict:
-        """The failure words of the scratch set of batch size B (default: all sets), one small D2H each."""
+        """The failure words of the scratch set of batch size B (default: all sets) and of the native prompt passes, one small
+        D2H each."""
         out = {"attn_status": 0, "kv_oob": 0}
-        for b, s in self._scratch.items():
-            if B is None or b == B or (isinstance(b, tuple) and b[0] == B):
-                st, oob = s["flags"].tolist()
-                out["attn_status"] |= st
-                out["kv_oob"] += oob
+        for f in self._flags(B):
+            st, oob = f.tolist()
+            out["attn_status"] |= st
+            out["kv_oob"] += oob
         return out
 
     def check_status(self, B: int | None = None) -> dict:
@@ -301,9 +315,8 @@ class DecodeEngine:
         a launch whose attention status bit is set are undefined, and a skipped KV write corrupts later tokens."""
         d = self.device_status(B)
         if d["attn_status"] or d["kv_oob"]:
-            for b, s in self._scratch.items():
-                if B is None or b == B or (isinstance(b, tuple) and b[0] == B):
-                    s["flags"].zero_()
+            for f in self._flags(B):
+                f.zero_()
             raise _lib.UvError(f"decode kernels reported a device-side failure: attention status word "
                                f"{d['attn_status']:#x} (bit 0 = a cache tile copy timed out, bit 3 = a wait inside the one-launch step), {d['kv_oob']} KV "
                                "cache writes skipped as out of range; tokens produced since the last check are invalid")
@@ -373,7 +386,7 @@ class DecodeEngine:
                     _lib.check(lib.uv_decode_step(C.byref(a), sp), "uv_decode_step")
                     return s["xn"]
         if self.tc_gemm and not fused and not qkv_in_attn and B <= self.BIG_ROWS:
-            return self._trunk_tc(tok, st, pos, starts, g_len, ns, rm, row_map, skip_attn, packed)
+            return self._trunk_tc(tok, st, pos, starts, g_len, ns, rm, row_map, skip_attn, packed, scratch_tag)
         with torch.cuda.device(self.device):
             use_table = self.rope_table and not fused and cfg.rope_pairs > 0
             if use_table:  # one cos / sin table per step instead of cosf / sinf in every layer's prologue
@@ -512,13 +525,13 @@ class DecodeEngine:
         a.xn, a.oob_count, a.status, a.h_layers = s["xn"].data_ptr(), s["oob"].data_ptr(), s["status"].data_ptr(), layers
         return a
 
-    def _trunk_tc(self, tok, st, pos, starts, g_len, ns, rm, row_map, skip_attn, packed) -> Tensor:
+    def _trunk_tc(self, tok, st, pos, starts, g_len, ns, rm, row_map, skip_attn, packed, scratch_tag) -> Tensor:
         """The step on the tensor-core GEMM path: per layer  uv_gemm_sw_qkv -> attention -> uv_gemm_sw_resid (wo) ->
         uv_gemm_sw_swiglu -> uv_gemm_sw_resid (down); the residual stream stays un-normalised and every consumer
         applies the RMS norm to its own result (per-tile sums of squares travel in ss_x / ss_h)."""
         cfg, lib, dt = self.cfg, _lib.lib(), DTYPE_CODE[self.dtype]
         B = tok.size(0)
-        s = self.scratch(B)
+        s = self.scratch(B, scratch_tag)
         d, hd, H, K, f = cfg.d_model, cfg.head_dim, cfg.n_heads, cfg.n_kv_heads, cfg.d_ff
         sp = stream_ptr(self.device)
         w = self.w

@@ -167,12 +167,11 @@ def prefill_packed(eng, st, idx: Tensor, starts: Tensor, rows: Tensor, lens_h) -
     if trunk is not None and idx.dtype == torch.int64 and idx.stride(1) == 1:
         lens = np.asarray(lens_h, dtype=np.int64)
         M = int(lens.sum())
-        s = eng.scratch(M)
-        return trunk.run(idx, starts, rows, M, int(((lens + 15) // 16).sum()), s["x"], s["xn"], s["qkv"], s["z"], s["gu"],
-                         s["act"], s["gate"], s["rope_cs"], s["oob"], st.k, st.v, st.k_scale, st.v_scale)
+        return trunk.run(idx, starts, rows, M, int(((lens + 15) // 16).sum()), eng.prefill_oob(), st.k, st.v, st.k_scale, st.v_scale)
     pk = pack_prompts(idx, starts, rows, lens_h)
     zero = torch.zeros(pk["M"], dtype=torch.int64, device=idx.device)
-    h = eng.trunk(pk["tok"], st, pk["pos"], zero, g_len=idx.size(1), row_map=pk["rows"], packed=pk)
+    h = eng.trunk(pk["tok"], st, pk["pos"], zero, g_len=idx.size(1), row_map=pk["rows"], packed=pk,
+                  scratch_tag="prefill")
     out = h[pk["last_row"]]
     return out.masked_fill(pk["empty"][:, None], 0)
 
