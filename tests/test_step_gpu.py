@@ -84,3 +84,12 @@ def test_one_launch_against_single_kernels(dtype, B, max_len, over):
             assert d.max() <= (2 if l == 0 else 12) and (d > 1).float().mean() < 1e-3
         for p, q in ((sa.k_scale[l], sb.k_scale[l]), (sa.v_scale[l], sb.v_scale[l])):
             assert torch.allclose(p.float(), q.float(), rtol=4 * tol, atol=0)
+
+
+def test_launch_count():
+    m = _model(torch.bfloat16, vocab_size=300, n_layers=2)
+    eng, st = m.engine, m.new_state(300, 40)
+    assert eng.launches_per_step(st, 1) == eng.launches_per_step(st, 48) == 2
+    assert eng.launches_per_step(st) == eng.launches_per_step(st, 256) == eng.launches_per_step() == 1 + 7 * 2 + 2
+    eng.one_launch = False
+    assert eng.launches_per_step(st, 1) == 17

@@ -322,9 +322,16 @@ class DecodeEngine:
                                "cache writes skipped as out of range; tokens produced since the last check are invalid")
         return d
 
-    def launches_per_step(self) -> int:
-        """Kernel launches of one trunk + head call (the sampler is one more).  A batch that uv_decode_step takes has one
-        launch for all layers."""
+    def launches_per_step(self, st=None, B: int | None = None) -> int:
+        """Kernel launches of one trunk + head call (the sampler is one more).  With the decode state: of a step of its first B
+        rows (default: all), which is one launch and the head where uv_decode_step takes them; without: of one launch per
+        operation, as batches too large for that and a scheduler's steps run."""
+        if st is not None and self.one_launch:
+            B = B or st.B
+            with torch.cuda.device(self.device):
+                a = self._step_args(st.pos[:B], st, st.pos, st.starts, None, self.scratch(B))
+                if _lib.lib().uv_decode_step_supported(C.byref(a)):
+                    return 2
         n = self.cfg.n_layers
         if self.tc_gemm:
             return 1 + 5 * n + 2
