@@ -1,5 +1,5 @@
 """All layers of a decode step in one launch (uv_decode_step) against one launch per operation: hidden states, appended
-cache entries and the count of skipped writes after several steps.  Batches around the row tiles, mixed contexts (a single
+cache entries and the count of skipped writes after several steps, and the tokens sampled from them.  Batches around the row tiles, mixed contexts (a single
 key, ends inside a chunk, ring caches before and after they wrap, a position past the cache), remapped cache rows, models
 with fewer heads, odd gate widths, other rotation widths and features left out."""
 import pytest
@@ -74,16 +74,68 @@ def test_one_launch_against_single_kernels(dtype, B, max_len, over):
         res.append((out, st, eng.device_status(B)))
         eng.scratch(B)["flags"].zero_()
     (xs, sa, fa), (ys, sb, fb) = res
-    tol = 3e-2 if dtype == torch.bfloat16 else 5e-3
+    # twice what was measured on these cases: hidden states (norm, largest value) of ten layers 7.5e-3, 1.8e-2 in bf16 and
+    # 1.5e-3, 3.9e-3 in fp16, of two or three layers at most a quarter of that; scales 1.6e-2 and 2.7e-3; bytes by 1 in the
+    # first layer and 3 in later ones, by more than 1 in 1.8e-4 of them
+    norm, most, scale = (1.5e-2, 3.6e-2, 3.2e-2) if dtype == torch.bfloat16 else (3e-3, 8e-3, 5.4e-3)
+    part = 1.0 if cfg.n_layers == 10 else 0.3
     for x, y in zip(xs, ys):
-        assert (x - y).norm() <= tol * y.norm() and (x - y).abs().max() <= 4 * tol * y.abs().max()
+        assert (x - y).norm() <= part * norm * y.norm() and (x - y).abs().max() <= part * most * y.abs().max()
     assert fa["attn_status"] == fb["attn_status"] == 0 and fa["kv_oob"] == fb["kv_oob"]
     for l in range(cfg.n_layers):
         for p, q in ((sa.k[l], sb.k[l]), (sa.v[l], sb.v[l])):
             d = (p.int() - q.int()).abs()
-            assert d.max() <= (2 if l == 0 else 12) and (d > 1).float().mean() < 1e-3
+            assert d.max() <= (1 if l == 0 else 6) and (d > 1).float().mean() < 4e-4
         for p, q in ((sa.k_scale[l], sb.k_scale[l]), (sa.v_scale[l], sb.v_scale[l])):
-            assert torch.allclose(p.float(), q.float(), rtol=4 * tol, atol=0)
+            assert torch.allclose(p.float(), q.float(), rtol=scale, atol=0)
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "fp16"])
+@pytest.mark.parametrize("temperature,top_p,other", [(0.0, 1.0, 0.002), (0.8, 0.95, 0.002), (1.0, 1.0, 0.02)])
+def test_sampled_tokens(dtype, temperature, top_p, other):
+    """Tokens and log-probs of DecodeRunner steps of a trained-like policy, both kinds of step.  Measured over 19,000 tokens: greedy
+    and nucleus draws are the same tokens, untruncated draws at T = 1 others in 0.4 % (a sequence that took another token
+    goes on from there); log-probs up to there by 1.1e-3 at most in bf16 and 2.3e-4 in fp16, 1.5e-5 and 1.5e-6 in the mean."""
+    from perf import cases
+    m = cases._model(dtype)
+    differ, total, logp = 0, 0, []
+    for batch, seed in ((8, 0), (48, 0), (48, 1), (37, 2)):
+        case = dict(kind="step", batch=batch, lo=100, hi=500, steps=6, temperature=temperature, top_p=top_p, dtype=dtype)
+        res = []
+        for one in (True, False):
+            m.engine.one_launch = one
+            try:
+                r = cases.run(cases.prepare(case, seed))
+            finally:
+                m.engine.one_launch = True
+            res.append((r["tok"].clone(), r["logp"].clone()))
+        d = res[0][0] != res[1][0]
+        differ, total = differ + int(d.sum()), total + d.numel()
+        logp.append((res[0][1] - res[1][1]).abs()[~d.cummax(0).values])
+    logp = torch.cat(logp)
+    assert differ <= other * total
+    # (an untruncated draw can land in the tail, whose log-probs of -16 move by 0.18 at most in bf16 -- test_fixed_tokens in
+    # test_rollout_step_gpu.py -- and by an eighth of that in fp16, as the hidden states do; twice of it is allowed)
+    tail = temperature == 1.0
+    assert logp.max() <= (0.36 if dtype == "bf16" else 0.05) if tail else logp.max() <= (2.2e-3 if dtype == "bf16" else 4.6e-4)
+    assert tail or logp.mean() <= (3e-5 if dtype == "bf16" else 3e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("B", [1, 8, 17, 48, 64, 256])
+@pytest.mark.parametrize("K", [512, 1664])
+def test_library_rounds_the_product_before_the_sum(dtype, B, K):
+    """What the one-launch step imitates in its residual adds: ``x.addmm_(z, w^T)`` rounds z w^T to the activation type and then the
+    sum.  Seen where that differs from one rounding (a quarter of the values).  Measured over batches of 1 to 512: up to 0.6 % of
+    those are otherwise, products that the order of the sum moves across a rounding edge; twice of it is allowed, and 4 values
+    for the scatter of a count of 0.6 % of 160 (two standard deviations over it is 3)."""
+    g = torch.Generator(device="cuda").manual_seed(B + K)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    w, z, x = (rnd(640, K) * 0.02).to(dtype), rnd(B, K).to(dtype), rnd(B, 640).to(dtype)
+    got, p = x.clone().addmm_(z, w.t()), z.double() @ w.double().t()
+    two, one = (x.double() + p.to(dtype).double()).to(dtype), (x.double() + p).to(dtype)
+    seen = two != one
+    assert seen.float().mean() > 0.15 and (got != two)[seen].sum() <= 0.012 * seen.sum() + 4
 
 
 def test_launch_count():
