@@ -54,3 +54,23 @@ def test_parameters_it_cannot_take_and_lambdas_it_cannot_fold():
     m.blocks[2].resid_mlp.data.fill_(1e-3)
     with pytest.raises(ValueError, match="layer 2"):
         eng.load_from(m)
+
+
+@pytest.mark.parametrize("name,shape", [("wq", (40, 64)), ("wk", (64, 32)), ("attn_gate", (4, 8)), ("xsa_alpha", (2,)),
+                                        ("o_scale", (1,)), ("embed", (500, 64)), ("value_embed", (512, 16))])
+def test_shapes_that_are_not_the_configs(name, shape):
+    """Parameters of other shapes are not for the launch, which reads them by the config's: they go to the tensor operations, which
+    take or refuse them."""
+    from ultraviolet_b200.engine import DecodeEngine
+    m = _model({}, torch.float32)
+    eng = DecodeEngine.from_model(m, torch.bfloat16)
+    at = m.blocks[1].attn
+    p = getattr(m, name).weight if "embed" in name else getattr(at, name)
+    assert p.shape != shape
+    p.data = torch.ones(shape, device="cuda")
+    if name == "o_scale":
+        eng.load_from(m)
+    else:
+        with pytest.raises(RuntimeError):
+            eng.load_from(m)
+    assert eng._fuse_plan["args"] is None

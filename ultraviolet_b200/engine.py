@@ -145,7 +145,8 @@ class DecodeEngine:
     def load_from(self, model) -> None:
         """(Re)compute every fused weight from the model's parameters INTO the existing arena (same formulas and
         rounding as Attention.fuse / MLP.fuse; pointers never change).  One launch (uv_fuse_weights) where the
-        parameters are contiguous tensors of one dtype on this device, tensor operations otherwise."""
+        parameters are contiguous tensors of one dtype and of the config's shapes on this device, tensor operations
+        otherwise."""
         if not self._fuse_launch(model):
             self._fuse_by_tensor_ops(model)
         self.version += 1
@@ -177,30 +178,35 @@ class DecodeEngine:
         dt = model.embed.weight.dtype
         ok = dt in (torch.float32, torch.float16, torch.bfloat16) and cfg.n_layers <= 32
 
-        def src(t):
+        def src(t, *shape):
             nonlocal ok
-            ok = ok and torch.is_tensor(t) and t.dtype == dt and t.device == self.arena.device and t.is_contiguous()
+            ok = (ok and type(t) in (Tensor, torch.nn.Parameter) and t.dtype == dt and t.device == self.arena.device
+                  and t.shape == shape and t.is_contiguous())
             return t.data_ptr() if ok else None
+        d, q, kv, f = cfg.d_model, cfg.n_heads * cfg.head_dim, cfg.n_kv_heads * cfg.head_dim, cfg.d_ff
         layers = (_lib.FuseLayer * cfg.n_layers)()
         for l, (blk, y) in enumerate(zip(model.blocks, layers)):
             at, mlp = blk.attn, blk.mlp
-            y.wq, y.wk, y.wv, y.wo = src(at.wq), src(at.wk), src(at.wv), src(at.wo)
-            y.w_gate, y.w_up, y.w_down = src(mlp.w_gate), src(mlp.w_up), src(mlp.w_down)
+            y.wq, y.wk, y.wv, y.wo = src(at.wq, q, d), src(at.wk, kv, d), src(at.wv, kv, d), src(at.wo, d, q)
+            y.w_gate, y.w_up, y.w_down = src(mlp.w_gate, f, d), src(mlp.w_up, f, d), src(mlp.w_down, d, f)
             y.qkv_scale, y.o_scale = src(at.qkv_scale), src(at.o_scale)
             y.resid_attn, y.post_attn = src(blk.resid_attn), src(blk.post_attn)
             y.resid_mlp, y.post_mlp = src(blk.resid_mlp), src(blk.post_mlp)
             y.d_wqkv, y.d_wo, y.d_gu, y.d_down = (w[f"l{l}.{n}"].data_ptr() for n in ("wqkv", "wo", "gu", "down"))
             y.d_lambdas = self.lambdas[l].data_ptr()
             if cfg.has_ve(l):
-                y.ve_gate, y.d_ve_gate = src(at.ve_gate), w[f"l{l}.ve_gate"].data_ptr()
+                y.ve_gate = src(at.ve_gate, cfg.n_kv_heads, cfg.ve_gate_channels)
+                y.d_ve_gate = w[f"l{l}.ve_gate"].data_ptr()
             if cfg.gate_channels:
-                y.attn_gate, y.d_attn_gate = src(at.attn_gate), w[f"l{l}.attn_gate"].data_ptr()
+                y.attn_gate = src(at.attn_gate, cfg.n_heads, cfg.gate_channels)
+                y.d_attn_gate = w[f"l{l}.attn_gate"].data_ptr()
             if cfg.xsa:
-                y.xsa_alpha, y.d_xsa = src(at.xsa_alpha), self.xsa[l].data_ptr()
+                y.xsa_alpha, y.d_xsa = src(at.xsa_alpha, cfg.n_heads), self.xsa[l].data_ptr()
         a = _lib.FuseArgs()
-        a.embed, a.d_embed = src(model.embed.weight), w["embed"].data_ptr()
+        a.embed, a.d_embed = src(model.embed.weight, cfg.vocab_size, d), w["embed"].data_ptr()
         if self.use_ve:
-            a.value_embed, a.d_value_embed = src(model.value_embed.weight), w["value_embed"].data_ptr()
+            a.value_embed = src(model.value_embed.weight, cfg.vocab_size, kv)
+            a.d_value_embed = w["value_embed"].data_ptr()
         if not ok or len(model.blocks) != cfg.n_layers:
             return plan
         a.src_dtype, a.dst_dtype, a.n_layers, a.fold = DTYPE_CODE[dt], DTYPE_CODE[self.dtype], cfg.n_layers, int(self.fold)
