@@ -74,3 +74,43 @@ def test_shapes_that_are_not_the_configs(name, shape):
         with pytest.raises(RuntimeError):
             eng.load_from(m)
     assert eng._fuse_plan["args"] is None
+
+
+def test_same_memory_other_form():
+    """Parameters that come back in the same memory with another shape, order or type are looked at again."""
+    from ultraviolet_b200.engine import DecodeEngine
+    m = _model(dict(d_model=64, n_heads=4, head_dim=16), torch.float32)         # wq and wo are square
+    eng = DecodeEngine.from_model(m, torch.bfloat16)
+    eng.load_from(m)
+    plan = eng._fuse_plan
+    eng.load_from(m)
+    assert eng._fuse_plan is plan and plan["args"] is not None
+    at = m.blocks[2].attn
+    at.wq.data = at.wq.data.t()
+    eng.load_from(m)
+    got = eng.arena.clone()
+    with torch.no_grad():
+        eng._fuse_by_tensor_ops(m)
+    assert torch.equal(got, eng.arena) and eng._fuse_plan["args"] is None
+    at.wq.data = at.wq.data.t()
+    eng.load_from(m)
+    assert eng._fuse_plan["args"] is not None
+    at.wk.data = at.wk.data.reshape(-1)
+    with pytest.raises((RuntimeError, ValueError)):
+        eng.load_from(m)
+
+
+def test_parametrised_weight():
+    from ultraviolet_b200.engine import DecodeEngine
+    m = _model({}, torch.float32)
+    eng = DecodeEngine.from_model(m, torch.bfloat16)
+
+    class Double(torch.nn.Module):
+        def forward(self, w):
+            return 2 * w
+    torch.nn.utils.parametrize.register_parametrization(m.blocks[0].attn, "wv", Double())
+    eng.load_from(m)
+    got = eng.arena.clone()
+    with torch.no_grad():
+        eng._fuse_by_tensor_ops(m)
+    assert torch.equal(got, eng.arena) and eng._fuse_plan["args"] is None

@@ -188,6 +188,45 @@ void gemm(int M, const void* x, const Tensor& w, void* c, bool accumulate = fals
   TORCH_CHECK(s == CUBLAS_STATUS_SUCCESS, "cublasGemmEx failed with status ", (int)s);
 }
 
+// ---- what a prepared launch over a list of tensors was prepared for: their memory, types, sizes and strides
+class TensorFacts {
+ public:
+  explicit TensorFacts(const std::vector<Tensor>& ts) {
+    for (const Tensor& t : ts)
+      facts_.push_back({t.const_data_ptr(), t.scalar_type(), t.device(), t.sizes().vec(), t.strides().vec(), plain(t), t.is_contiguous()});
+  }
+  bool match(const std::vector<Tensor>& ts) const {
+    if (ts.size() != facts_.size()) return false;
+    for (size_t i = 0; i < ts.size(); ++i) {
+      const Fact& f = facts_[i];
+      const Tensor& t = ts[i];
+      if (!f.plain || !plain(t) || t.const_data_ptr() != f.data || t.scalar_type() != f.type || t.device() != f.device ||
+          t.sizes() != f.sizes || t.strides() != f.strides)
+        return false;
+    }
+    return true;
+  }
+  // all of them contiguous, of one type, on t's device
+  bool uniform_with(const Tensor& t) const {
+    for (const Fact& f : facts_)
+      if (!f.plain || !f.contiguous || f.type != facts_[0].type || f.device != t.device()) return false;
+    return !facts_.empty();
+  }
+
+ private:
+  struct Fact {
+    const void* data;
+    at::ScalarType type;
+    c10::Device device;
+    std::vector<int64_t> sizes, strides;
+    bool plain, contiguous;
+  };
+  static bool plain(const Tensor& t) {
+    return t.layout() == at::kStrided && !t.unsafeGetTensorImpl()->key_set().has(c10::DispatchKey::Python);
+  }
+  std::vector<Fact> facts_;
+};
+
 // ---- one packed prompt pass through every layer (DecodeEngine.trunk with packed=..., folded stream)
 struct LayerFacts {
   Tensor wqkv, wo, gu, down;
@@ -292,6 +331,10 @@ PYBIND11_MODULE(_uvhost, m) {
   m.def("init", &init);
   m.def("decode_attention", &decode_attention);
   m.def("fused_sample", &fused_sample);
+  py::class_<TensorFacts>(m, "TensorFacts")
+      .def(py::init<const std::vector<Tensor>&>())
+      .def("match", &TensorFacts::match)
+      .def("uniform_with", &TensorFacts::uniform_with);
   py::class_<PrefillTrunk>(m, "PrefillTrunk")
       .def(py::init<std::vector<Tensor>, std::vector<Tensor>, std::vector<Tensor>, std::vector<Tensor>, std::vector<int64_t>,
                     std::vector<int64_t>, std::vector<int64_t>, std::vector<bool>, std::vector<bool>, std::vector<int64_t>,

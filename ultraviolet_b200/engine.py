@@ -17,7 +17,6 @@ from __future__ import annotations
 
 import ctypes as C
 import os
-import weakref
 
 import torch
 from torch import Tensor
@@ -158,11 +157,9 @@ class DecodeEngine:
         params = [model.embed.weight, model.value_embed.weight if self.use_ve else None]
         params += [q for m in mods for q in m._parameters.values()]
         params = [q for q in params if q is not None]
-        ptrs = [q.data_ptr() for q in params]
         plan = self._fuse_plan
-        if (plan is None or plan["ptrs"] != ptrs or plan["fold"] != self.fold
-                or any(r() is not q for r, q in zip(plan["refs"], params))):
-            plan = self._fuse_plan = self._plan_fuse(model, ptrs, [weakref.ref(q) for q in params])
+        if plan is None or plan["fold"] != self.fold or not plan["facts"].match(params):
+            plan = self._fuse_plan = self._plan_fuse(model, params, _lib.host().TensorFacts(params))
         if plan["args"] is None:
             return False
         with torch.cuda.device(self.device):
@@ -170,18 +167,18 @@ class DecodeEngine:
             _lib.check(_lib.lib().uv_fuse_weights(C.byref(plan["args"]), stream_ptr(self.device)), "uv_fuse_weights")
         return not self.fold or int(self._fuse_status.item()) == 0
 
-    def _plan_fuse(self, model, ptrs, refs) -> dict:
-        """Arguments of uv_fuse_weights for these parameter tensors (kept as long as the same tensors come back:
-        walking a few hundred attributes costs more than the kernel)."""
+    def _plan_fuse(self, model, params, facts) -> dict:
+        """Arguments of uv_fuse_weights for these parameter tensors (kept as long as tensors of the same memory, types, sizes
+        and strides come back: walking a few hundred attributes costs more than the kernel)."""
         cfg, w = self.cfg, self.w
-        plan = dict(ptrs=ptrs, refs=refs, fold=self.fold, args=None)
+        plan = dict(facts=facts, fold=self.fold, args=None)
         dt = model.embed.weight.dtype
-        ok = dt in (torch.float32, torch.float16, torch.bfloat16) and cfg.n_layers <= 32
+        ok = dt in (torch.float32, torch.float16, torch.bfloat16) and cfg.n_layers <= 32 and facts.uniform_with(self.arena)
+        known = {id(t) for t in params}     # (a parametrised weight is computed anew each time it is asked for)
 
         def src(t, *shape):
             nonlocal ok
-            ok = (ok and type(t) in (Tensor, torch.nn.Parameter) and t.dtype == dt and t.device == self.arena.device
-                  and t.shape == shape and t.is_contiguous())
+            ok = ok and id(t) in known and t.shape == shape
             return t.data_ptr() if ok else None
         d, q, kv, f = cfg.d_model, cfg.n_heads * cfg.head_dim, cfg.n_kv_heads * cfg.head_dim, cfg.d_ff
         layers = (_lib.FuseLayer * cfg.n_layers)()
