@@ -145,3 +145,28 @@ def test_prefill_keeps_no_buffers_per_length(native, monkeypatch):
         assert eng.device_status() == {"attn_status": 0, "kv_oob": 0}
     else:
         assert sorted(k[0] for k in eng._scratch) == [64, 128, 1024, 2048, 4096]        # (1 ... 127, 1000, 2048, 2049, 2150)
+
+
+def test_prefill_into_strided_rows_and_what_it_refuses():
+    from ultraviolet_b200.model import MathLM, make_config
+    torch.manual_seed(7)
+    with torch.device("cuda"):
+        m = MathLM(make_config("uv-50m-alpha", vocab_size=500, n_layers=2)).bfloat16().fuse_for_inference()
+    idx, starts = torch.randint(1, 500, (3, 20), device="cuda"), torch.tensor([0, 5, 19], device="cuda")
+    rows = torch.tensor([[6, 0], [1, 0], [4, 0]], device="cuda")
+    res = []
+    for r, s in ((rows[:, 0], starts), (torch.tensor([6, 1, 4], device="cuda"), starts),
+                 (rows[:, 0].int(), torch.stack([starts, starts], 1)[:, 1].int())):
+        st = m.new_state(8, 24)
+        res.append((m.prefill(idx, s, st, rows=r), st.pos, st.starts, *st.k, *st.v))
+    for other in res[1:]:
+        for a, b in zip(res[0], other):
+            assert torch.equal(a, b)
+    st, good = m.new_state(8, 24), torch.tensor([6, 1, 4], device="cuda")
+    for bad in (dict(rows=good[:2]), dict(rows=good[:, None]), dict(starts=starts[:1]), dict(starts=torch.zeros(4).cuda().long())):
+        with pytest.raises(ValueError):
+            m.prefill(idx, bad.get("starts", starts), st, rows=bad.get("rows", good))
+    for bad in (dict(rows=good.cpu()), dict(starts=starts.cpu()), dict(idx=idx.cpu())):
+        with pytest.raises(RuntimeError):
+            m.prefill(bad.get("idx", idx), bad.get("starts", starts), st, rows=bad.get("rows", good))
+    assert not any(k.any() for k in st.k)

@@ -108,7 +108,11 @@ def prefill_fast(self, idx: Tensor, starts: Tensor, st: KernelDecodeState, rows:
         if n != st.B:
             raise AssertionError("prefill without rows needs one prompt per cache row")
         rows = torch.arange(n, device=dev)
-    rows = rows.to(torch.int64)
+    if rows.shape != (n,) or starts.shape != (n,):
+        raise ValueError("prefill takes one cache row and one start per prompt")
+    if not dev == rows.device == starts.device == eng.arena.device:
+        raise RuntimeError(f"prefill takes its prompts, starts and rows on {eng.arena.device}")
+    rows = rows.to(torch.int64).contiguous()
     starts = starts.to(torch.int64).contiguous()
     # the one host round trip (the reference has one too, :111)
     lens_h = np.clip(T - starts.cpu().numpy(), 0, T)
