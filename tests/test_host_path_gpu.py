@@ -170,3 +170,34 @@ def test_prefill_into_strided_rows_and_what_it_refuses():
         with pytest.raises(RuntimeError):
             m.prefill(bad.get("idx", idx), bad.get("starts", starts), st, rows=bad.get("rows", good))
     assert not any(k.any() for k in st.k)
+
+
+def test_watched_attention_calls_go_through_the_op():
+    """Tracers, transforms and subclasses see the custom op, not a result computed behind their back."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from ultraviolet_b200.kernels import decode_attention
+    g = torch.Generator(device="cuda").manual_seed(0)
+
+    def inputs():
+        q = torch.randn(4, 8, 64, device="cuda", generator=g).half()
+        k, v = (torch.randint(-127, 128, (4, 1, 64, 64), device="cuda", generator=g, dtype=torch.int8) for _ in range(2))
+        ks, vs = (torch.rand(4, 1, 64, device="cuda", generator=g).half() * 0.02 for _ in range(2))
+        return q, k, v, torch.full((4,), 50, device="cuda"), torch.zeros(4, dtype=torch.long, device="cuda"), ks, vs
+
+    def f(q, k, v, pos, starts, ks, vs):
+        return decode_attention(q, k, v, pos, starts, 0.1, k_scale=ks, v_scale=vs, num_splits=1)
+    a, b = inputs(), inputs()
+    want = f(*b)
+    assert torch.equal(torch.jit.trace(f, a, check_trace=False)(*b), want)
+    for pre in (False, True):
+        assert torch.equal(make_fx(f, pre_dispatch=pre)(*a)(*b), want)
+    assert torch.equal(torch.func.vmap(f)(*(torch.stack(t) for t in zip(a, b)))[1], want)
+    seen = []
+
+    class Watch(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return super().__torch_function__(func, types, args, kwargs or {})
+    f(b[0].as_subclass(Watch), *b[1:])
+    assert any("decode_attn" in n for n in seen)

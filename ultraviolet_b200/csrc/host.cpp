@@ -2,6 +2,7 @@
 // (ultraviolet_b200._uvhost): reading tensor metadata, filling argument blocks and launching through libuvdecode's C ABI.
 // Each function returns None for arguments it does not take as they are (other devices or layouts, tensor subclasses,
 // dispatch modes); the caller's Python then handles or rejects them.
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -86,12 +87,22 @@ int code_of(at::ScalarType t) {
 
 // a tensor whose metadata and memory can be taken at face value on CUDA device `dev`
 bool plain(const Tensor& t, c10::Device dev) {
-  return t.defined() && t.device() == dev && !t.unsafeGetTensorImpl()->key_set().has(c10::DispatchKey::Python) &&
-         t.layout() == at::kStrided && !(t.requires_grad() && at::GradMode::is_enabled());
+  const c10::DispatchKeySet keys = t.unsafeGetTensorImpl()->key_set();
+  return t.defined() && t.device() == dev && t.layout() == at::kStrided && !keys.has(c10::DispatchKey::Python) &&
+         !keys.has(c10::DispatchKey::Functionalize) && !(t.requires_grad() && at::GradMode::is_enabled()) &&
+         !t._fw_grad(0).defined();
 }
+// nothing watches or rewrites the calls of this thread: no dispatch or function mode, transform or tracer
 bool modes_off() {
-  return !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
-         !c10::impl::tls_local_dispatch_key_set().included_.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+  constexpr c10::DispatchKeySet watchers({c10::DispatchKey::FuncTorchDynamicLayerFrontMode, c10::DispatchKey::Tracer,
+                                          c10::DispatchKey::Functionalize, c10::DispatchKey::PreDispatch,
+                                          c10::DispatchKey::Python, c10::DispatchKey::PythonDispatcher});
+  return !c10::impl::TorchDispatchModeTLS::any_modes_set() && !at::impl::torch_function_mode_enabled() &&
+         !c10::impl::tls_local_dispatch_key_set().included_.has_any(watchers);
+}
+// the tensor of a Python object that is a torch.Tensor or a parameter, not one of a subclass; else null
+const Tensor* exact(py::handle h) {
+  return THPVariable_CheckExact(h.ptr()) ? &THPVariable_Unpack(h.ptr()) : nullptr;
 }
 const void* ro(const Tensor& t) { return t.const_data_ptr(); }
 
@@ -114,9 +125,14 @@ int64_t row_alloc(const Tensor& k, const Tensor& v, const Tensor& ks, const Tens
 
 constexpr int64_t kAutoSplits = INT32_MIN;
 
-std::optional<Tensor> decode_attention(const Tensor& q_, const Tensor& k, const Tensor& v, const Tensor& pos,
-                                       const Tensor& starts, double scale, int64_t window, int64_t ring,
-                                       const Tensor& ks, const Tensor& vs, int64_t ctx, int64_t splits) {
+std::optional<Tensor> decode_attention(py::handle hq, py::handle hk, py::handle hv, py::handle hpos, py::handle hstarts,
+                                       double scale, int64_t window, int64_t ring, py::handle hks, py::handle hvs,
+                                       int64_t ctx, int64_t splits) {
+  const Tensor* in[7];
+  const py::handle from[7] = {hq, hk, hv, hpos, hstarts, hks, hvs};
+  for (int i = 0; i < 7; ++i)
+    if (!(in[i] = exact(from[i]))) return std::nullopt;
+  const Tensor &q_ = *in[0], &k = *in[1], &v = *in[2], &pos = *in[3], &starts = *in[4], &ks = *in[5], &vs = *in[6];
   if (!q_.is_cuda() || !modes_off()) return std::nullopt;
   const c10::Device dev = q_.device();
   for (const Tensor* t : {&q_, &k, &v, &pos, &starts, &ks, &vs})
@@ -158,8 +174,11 @@ std::optional<Tensor> decode_attention(const Tensor& q_, const Tensor& k, const 
 }
 
 // ---- kernels.fused_sample
-std::optional<std::pair<Tensor, Tensor>> fused_sample(const Tensor& x, const Tensor& u, double a, double b, double c,
+std::optional<std::pair<Tensor, Tensor>> fused_sample(py::handle hx, py::handle hu, double a, double b, double c,
                                                       double temperature, double top_p) {
+  const Tensor *px = exact(hx), *pu = exact(hu);
+  if (!px || !pu) return std::nullopt;
+  const Tensor &x = *px, &u = *pu;
   if (!x.is_cuda() || !modes_off() || !plain(x, x.device()) || !plain(u, x.device())) return std::nullopt;
   if (x.dim() != 2 || x.stride(1) != 1 || u.scalar_type() != at::kFloat || !u.is_contiguous() || u.numel() < x.size(0))
     return std::nullopt;
