@@ -201,3 +201,23 @@ def test_watched_attention_calls_go_through_the_op():
             return super().__torch_function__(func, types, args, kwargs or {})
     f(b[0].as_subclass(Watch), *b[1:])
     assert any("decode_attn" in n for n in seen)
+
+
+def test_logits_keep_gradients_and_transforms():
+    """MathLM.logits of hidden states that want gradients, or under a transform or tracer, is the tensor expression."""
+    from ultraviolet_b200.model import MathLM, make_config
+    torch.manual_seed(8)
+    with torch.device("cuda"):
+        m = MathLM(make_config("uv-50m-alpha", vocab_size=500, n_layers=1)).bfloat16().fuse_for_inference()
+    w, (a, b, c) = m.engine.w["embed"], m.cfg.softcap
+    h, t = torch.randn(2, 5, w.size(1), device="cuda").bfloat16()
+    ref = lambda x: a * torch.sigmoid((torch.mm(x, w.t()).float() + b) / c)
+    assert torch.allclose(m.logits(h), ref(h), rtol=1e-5, atol=1e-6)
+    x, y = h.clone().requires_grad_(), h.clone().requires_grad_()
+    got, want = m.logits(x), ref(y)
+    got.square().sum().backward(), want.square().sum().backward()
+    assert torch.equal(got, want) and torch.equal(x.grad, y.grad) and x.grad.any()
+    for p, q in zip(torch.func.jvp(m.logits, (h,), (t,)), torch.func.jvp(ref, (h,), (t,))):
+        assert torch.equal(p, q)
+    assert torch.equal(torch.func.vmap(m.logits)(torch.stack([h, t])), torch.func.vmap(ref)(torch.stack([h, t])))
+    assert torch.equal(torch.jit.trace(lambda x: m.logits(x), (h,), check_trace=False)(t), ref(t))

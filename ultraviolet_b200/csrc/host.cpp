@@ -104,6 +104,15 @@ bool modes_off() {
 const Tensor* exact(py::handle h) {
   return THPVariable_CheckExact(h.ptr()) ? &THPVariable_Unpack(h.ptr()) : nullptr;
 }
+// a call on these tensors may go to a kernel directly: contiguous memory on one CUDA device, no gradient wanted, nothing watching
+bool plain_call(const std::vector<py::object>& objects) {
+  if (!modes_off()) return false;
+  for (const py::object& o : objects) {
+    const Tensor* t = exact(o);
+    if (!t || !t->is_cuda() || !plain(*t, exact(objects[0])->device()) || !t->is_contiguous()) return false;
+  }
+  return true;
+}
 const void* ro(const Tensor& t) { return t.const_data_ptr(); }
 
 // ---- kernels.decode_attention on an int8 cache
@@ -348,6 +357,7 @@ class PrefillTrunk {
 
 PYBIND11_MODULE(_uvhost, m) {
   m.def("init", &init);
+  m.def("plain_call", &plain_call);
   m.def("decode_attention", &decode_attention);
   m.def("fused_sample", &fused_sample);
   py::class_<TensorFacts>(m, "TensorFacts")

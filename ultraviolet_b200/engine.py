@@ -655,7 +655,11 @@ class DecodeEngine:
         return self.softcap(torch.mm(h.to(self.dtype), self.w["embed"].t()))
 
     def softcap(self, head: Tensor) -> Tensor:
-        """fp32 softcapped logits of raw (B, V) head output."""
+        """fp32 softcapped logits of raw (B, V) head output: one launch, or tensor operations where a gradient is wanted or
+        something watches the call (a mode, a transform, a tracer)."""
+        if torch.compiler.is_compiling() or not _lib.host().plain_call([head]):
+            a, b, c = self.cfg.softcap
+            return a * torch.sigmoid((head.float() + b) / c)
         out = torch.empty(head.shape, dtype=torch.float32, device=head.device)
         with torch.cuda.device(self.device):
             _lib.check(_lib.lib().uv_softcap(head.data_ptr(), DTYPE_CODE[head.dtype], head.numel(), *self.cfg.softcap,
