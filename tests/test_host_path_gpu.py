@@ -170,6 +170,11 @@ def test_prefill_into_strided_rows_and_what_it_refuses():
         with pytest.raises(RuntimeError):
             m.prefill(bad.get("idx", idx), bad.get("starts", starts), st, rows=bad.get("rows", good))
     assert not any(k.any() for k in st.k)
+    for field in ("k", "v", "k_scale", "v_scale"):          # a state of a model with fewer layers
+        few = m.new_state(8, 24)
+        getattr(few, field).pop()
+        with pytest.raises(IndexError):
+            m.prefill(idx, starts, few, rows=good)
 
 
 def test_watched_attention_calls_go_through_the_op():

@@ -285,6 +285,9 @@ class PrefillTrunk {
   Tensor run(const Tensor& idx, const Tensor& starts, const Tensor& rows, int64_t M, int64_t max_tiles, Tensor oob,
              const std::vector<Tensor>& k, const std::vector<Tensor>& v, const std::vector<Tensor>& ks,
              const std::vector<Tensor>& vs) {
+    for (const auto* layers : {&k, &v, &ks, &vs})
+      TORCH_CHECK_INDEX(layers->size() >= layers_.size(), "the decode state has ", layers->size(), " layers, the model ",
+                        layers_.size());
     at::AutoDispatchBelowADInplaceOrView below;         // no autograd bookkeeping on the library calls below
     c10::cuda::CUDAGuard guard(embed_.device());
     void* st = at::cuda::getCurrentCUDAStream().stream();
