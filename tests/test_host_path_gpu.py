@@ -226,3 +226,23 @@ def test_logits_keep_gradients_and_transforms():
         assert torch.equal(p, q)
     assert torch.equal(torch.func.vmap(m.logits)(torch.stack([h, t])), torch.func.vmap(ref)(torch.stack([h, t])))
     assert torch.equal(torch.jit.trace(lambda x: m.logits(x), (h,), check_trace=False)(t), ref(t))
+
+
+def test_watched_prefill_shows_its_products():
+    from torch.utils.flop_counter import FlopCounterMode
+    from ultraviolet_b200.model import MathLM, make_config
+    torch.manual_seed(9)
+    with torch.device("cuda"):
+        m = MathLM(make_config("uv-50m-alpha", vocab_size=500, n_layers=2)).bfloat16().fuse_for_inference()
+    idx, starts = torch.randint(1, 500, (3, 20), device="cuda"), torch.tensor([0, 5, 19], device="cuda")
+    M, c = 20 + 15 + 1, m.cfg
+    d, q, kv, f = c.d_model, c.n_heads * c.head_dim, c.n_kv_heads * c.head_dim, c.d_ff
+    a, b = m.new_state(3, 24), m.new_state(3, 24)
+    want = m.prefill(idx, starts, a)
+    with FlopCounterMode(display=False) as count:
+        got = m.prefill(idx, starts, b)
+    # (QKV, gate | up and the head; the counter does not know the in-place addmm_ of the other two)
+    assert count.get_total_flops() == 2 * (c.n_layers * M * d * (q + 2 * kv + 2 * f) + 3 * d * 500)
+    assert torch.allclose(got, want, rtol=1e-5, atol=1e-6)
+    for x, y in zip(a.k + a.v + a.k_scale, b.k + b.v + b.k_scale):
+        assert torch.equal(x, y)

@@ -104,12 +104,12 @@ bool modes_off() {
 const Tensor* exact(py::handle h) {
   return THPVariable_CheckExact(h.ptr()) ? &THPVariable_Unpack(h.ptr()) : nullptr;
 }
-// a call on these tensors may go to a kernel directly: contiguous memory on one CUDA device, no gradient wanted, nothing watching
+// a call on these tensors may go to kernels directly: memory on one CUDA device, no gradient wanted, nothing watching
 bool plain_call(const std::vector<py::object>& objects) {
   if (!modes_off()) return false;
   for (const py::object& o : objects) {
     const Tensor* t = exact(o);
-    if (!t || !t->is_cuda() || !plain(*t, exact(objects[0])->device()) || !t->is_contiguous()) return false;
+    if (!t || !t->is_cuda() || !plain(*t, exact(objects[0])->device())) return false;
   }
   return true;
 }

@@ -657,7 +657,7 @@ class DecodeEngine:
     def softcap(self, head: Tensor) -> Tensor:
         """fp32 softcapped logits of raw (B, V) head output: one launch, or tensor operations where a gradient is wanted or
         something watches the call (a mode, a transform, a tracer)."""
-        if torch.compiler.is_compiling() or not _lib.host().plain_call([head]):
+        if torch.compiler.is_compiling() or not head.is_contiguous() or not _lib.host().plain_call([head]):
             a, b, c = self.cfg.softcap
             return a * torch.sigmoid((head.float() + b) / c)
         out = torch.empty(head.shape, dtype=torch.float32, device=head.device)

@@ -18,6 +18,7 @@ import numpy as np
 import torch
 from torch import Tensor
 
+from . import _lib
 from .config import MathConfig, config_from
 
 
@@ -166,9 +167,10 @@ def pack_prompts(idx: Tensor, starts: Tensor, rows: Tensor, lens_h) -> dict:
 def prefill_packed(eng, st, idx: Tensor, starts: Tensor, rows: Tensor, lens_h) -> Tensor:
     """One packed pass: returns the final normed hidden state of every prompt's last token (n, d) (zeros for an
     empty prompt).  The packing, the launches and the library calls of the pass are issued by the native host loop
-    (some 75 of them cost more from Python than they run for at a few dozen tokens)."""
+    (some 75 of them cost more from Python than they run for at a few dozen tokens), except where something watches the
+    call (a mode that counts operations, say) and has to see them."""
     trunk = eng.prefill_trunk()
-    if trunk is not None and idx.dtype == torch.int64 and idx.stride(1) == 1:
+    if trunk is not None and idx.dtype == torch.int64 and idx.stride(1) == 1 and _lib.host().plain_call([idx, starts, rows]):
         lens = np.asarray(lens_h, dtype=np.int64)
         M = int(lens.sum())
         return trunk.run(idx, starts, rows, M, int(((lens + 15) // 16).sum()), eng.prefill_oob(), st.k, st.v, st.k_scale, st.v_scale)
