@@ -26,6 +26,9 @@ def test_decode_attention_host_path(B, S, window, dtype, splits):
     want = _decode_attn_op(*args, window, window > 0, ks, vs, n)
     assert torch.equal(native, want)
     assert torch.equal(decode_attention(*args, window=window, k_scale=ks, v_scale=vs, num_splits=splits), want)
+    # numbers of any kind
+    assert torch.equal(decode_attention(*args[:5], torch.tensor(0.14, dtype=torch.float64), window=float(window), k_scale=ks,
+                                        v_scale=vs, num_splits=float(n), ctx_hint=float(S)), want)
     # what it does not take goes to the op: gradients wanted, other index types, a dispatch mode
     assert _lib.host().decode_attention(q.clone().requires_grad_(), k, v, pos, st, 0.14, window, -1, ks, vs, 0, 1) is None
     assert torch.equal(decode_attention(q, k, v, pos.int(), st, 0.14, window=window, k_scale=ks, v_scale=vs,

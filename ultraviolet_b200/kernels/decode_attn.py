@@ -143,9 +143,9 @@ def decode_attention(q: Tensor, k_cache: Tensor, v_cache: Tensor, pos: Tensor, s
     """
     if (not torch.compiler.is_compiling() and k_scale is not None and v_scale is not None
             and isinstance(pos, Tensor) and isinstance(starts, Tensor)):
-        out = _lib.host().decode_attention(q, k_cache, v_cache, pos, starts, scale, window,
-                                           -1 if ring is None else int(bool(ring)), k_scale, v_scale, ctx_hint or 0,
-                                           -2 ** 31 if num_splits is None else num_splits)
+        out = _lib.host().decode_attention(q, k_cache, v_cache, pos, starts, float(scale), int(window),
+                                           -1 if ring is None else int(bool(ring)), k_scale, v_scale, int(ctx_hint or 0),
+                                           -2 ** 31 if num_splits is None else int(num_splits))
         if out is not None:
             return out
     if q.dim() == 4:
