@@ -32,7 +32,8 @@
 // Rounding points are those of the per-kernel folded step (engine.py): projections round to the activation dtype, norms
 // scale the rounded projection, the residual stream adds it.
 //
-// Every wait is bounded (200 ms); a CTA that gives up sets status bit 3, skips its later waits and still ends.
+// Every wait is bounded (200 ms); a CTA that gives up sets status bit 3, skips its later waits for words (not those for its
+// own weight copies) and still ends.
 #include <mutex>
 #include <type_traits>
 
@@ -333,12 +334,16 @@ __device__ __forceinline__ void st_mma<__nv_bfloat16>(float (&d)[4], uint32_t a0
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// a wait that began at t_begin (0: just now) has taken too long, or another one has
-__device__ __forceinline__ bool st_late(unsigned long long& t_begin, volatile int* dead) {
+// a wait that began at t_begin (0: just now) has taken too long
+__device__ __forceinline__ bool st_late(unsigned long long& t_begin) {
   unsigned long long now;
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(now));
   if (t_begin == 0) t_begin = now;
-  if (!*dead && now - t_begin <= ST_WAIT_NS) return false;
+  return now - t_begin > ST_WAIT_NS;
+}
+// it has, or another one had
+__device__ __forceinline__ bool st_late(unsigned long long& t_begin, volatile int* dead) {
+  if (!*dead && !st_late(t_begin)) return false;
   *dead = 1;
   return true;
 }
@@ -401,7 +406,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) step_kernel(const __grid_consta
                  "l"(static_cast<const T*>(sm.layer[l].w[p]) + (int64_t)from * K), "r"(bytes), "r"(bar)
                  : "memory");
   };
-  auto weights_ready = [&](int p, int l) {              // of phase p, layer l
+  auto weights_ready = [&](int p, int l) {              // of phase p, layer l (also after another wait has given up: no CTA
+                                                        // may end with copies on their way to its memory)
     const uint32_t bar = smem_addr(&sm.full[p]);
     unsigned long long t_begin = 0;
 #pragma unroll 1
@@ -410,7 +416,10 @@ __global__ void __launch_bounds__(ST_THREADS, 1) step_kernel(const __grid_consta
       asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                    : "=r"(ok) : "r"(bar), "r"((uint32_t)(l & 1)) : "memory");
       if (ok) return;
-      if ((i & 63) == 63 && st_late(t_begin, dead)) return;
+      if ((i & 63) == 63 && st_late(t_begin)) {
+        *dead = 1;
+        return;
+      }
     }
   };
 
