@@ -268,9 +268,9 @@ __global__ void __launch_bounds__(SWR_THREADS) swiglu_rs_kernel(const T* __restr
 
 // The same for launches of many rows: a warp owns a row, requests all of it (16-byte pieces of h, g and u) before it
 // uses any, and forms rs once.  At prefill sizes the kernel above is bound by its own traffic -- four CTAs a row read
-// h four times and leave 48 bytes a thread in flight; this one streams.  20,500 rows of f = 1664: 99 us -> 43 us
-// (230 MB: 35 us at the measured copy rate; 49 back to back from the host).  The results are those of the kernel above bit for bit -- a row's bits must not
-// depend on how many rows came with it -- so the squares are summed in its order and the quotient is the rounded one.
+// h four times and leave 48 bytes a thread in flight; this one streams.  20,500 rows of f = 1664: 99 us -> 49 us (bf16; 45 in
+// fp16; 231 MB: 35 us at the measured copy rate).  The results are those of the kernel above bit for bit -- a row's bits must
+// not depend on how many rows came with it -- so the squares are summed in its order and the quotient is the rounded one.
 constexpr int SWM_WARPS = 8;
 constexpr int SWM_ROWS = 768;
 constexpr int SWM_V = 7;      // 8-feature vectors a lane holds at a time
