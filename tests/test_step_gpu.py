@@ -145,3 +145,26 @@ def test_launch_count():
     assert eng.launches_per_step(st) == eng.launches_per_step(st, 256) == eng.launches_per_step() == 1 + 7 * 2 + 2
     eng.one_launch = False
     assert eng.launches_per_step(st, 1) == 17
+
+
+@pytest.mark.parametrize("switches", [dict(fold=False), dict(fold=False, fused_gemm=True), dict(fold=False, tc_gemm=True),
+                                      dict(sw_qkv="1"), dict(qkv_in_attn=True)])
+def test_other_routes_are_not_replaced(switches):
+    """A batch of the one-launch step's sizes on an engine that was switched to another route takes that route."""
+    m = _model(torch.bfloat16, vocab_size=300, n_layers=3)
+    with torch.no_grad():
+        for b in m.blocks:
+            b.resid_attn.fill_(0.7), b.resid_mlp.fill_(1.3)
+    eng = m.engine
+    for name, value in switches.items():
+        setattr(eng, name, value)
+    eng.load_from(m)
+    tok = torch.arange(5, device="cuda") + 1
+    res = []
+    for one in (True, False):
+        st = m.new_state(5, 40)
+        res.append([eng.trunk(tok + i, st, st.pos + i, st.starts, g_len=40, one_launch=one).clone() for i in range(3)])
+        res[-1] += [*st.k, *st.v]
+    for a, b in zip(*res):
+        assert torch.equal(a, b)
+    assert eng.launches_per_step(st) == eng.launches_per_step()

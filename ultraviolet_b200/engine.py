@@ -291,6 +291,11 @@ class DecodeEngine:
             self._scratch[key] = s
         return s
 
+    def _one_launch_step(self) -> bool:
+        """Steps may take uv_decode_step: wanted, and the weights and the route are those of the plain folded step (the switches
+        may have been moved since the engine was made)."""
+        return self.one_launch and self.fold and self.sw_qkv == "0" and not (self.fused_gemm or self.tc_gemm or self.qkv_in_attn)
+
     def prefill_oob(self) -> Tensor:
         """The count of cache writes that native prompt passes skipped (their ``flags`` are those of a scratch set)."""
         if self._prefill_oob is None:
@@ -329,7 +334,7 @@ class DecodeEngine:
         """Kernel launches of one trunk + head call (the sampler is one more).  With the decode state: of a step of its first B
         rows (default: all), which is one launch and the head where uv_decode_step takes them; without: of one launch per
         operation, as batches too large for that and a scheduler's steps run."""
-        if st is not None and self.one_launch:
+        if st is not None and self._one_launch_step():
             B = B or st.B
             with torch.cuda.device(self.device):
                 a = self._step_args(st.pos[:B], st, st.pos, st.starts, None, self.scratch(B))
@@ -384,7 +389,7 @@ class DecodeEngine:
         fused = self.fused_gemm and packed is None
         qkv_in_attn = self.qkv_in_attn and packed is None
         fold = self.fold
-        if self.one_launch and one_launch and packed is None and not skip_attn and not shared_rows and not ns:
+        if one_launch and self._one_launch_step() and packed is None and not skip_attn and not shared_rows and not ns:
             with torch.cuda.device(self.device):
                 a = self._step_args(tok, st, pos, starts, rm, s)
                 if lib.uv_decode_step_supported(C.byref(a)):
@@ -669,7 +674,7 @@ class DecodeEngine:
     def prefill_trunk(self):
         """The native host loop of a packed prompt pass (None: this engine runs its trunk another way, or torch's matrix
         products are not the library call that the loop makes)."""
-        if not self.fold or self.sw_qkv != "0" or not self.rope_table or not default_matmul():
+        if not self.fold or self.sw_qkv != "0" or self.tc_gemm or not self.rope_table or not default_matmul():
             return None
         if self._prefill_trunk is None:
             cfg, w, L = self.cfg, self.w, range(self.cfg.n_layers)
