@@ -156,3 +156,14 @@ def test_default_matmul_sees_every_switch():
         finally:
             setattr(mm, name, before)
     assert default_matmul()
+
+
+def test_default_matmul_sees_deterministic_mode():
+    import torch
+    from ultraviolet_b200.engine import default_matmul
+    torch.use_deterministic_algorithms(True)
+    try:
+        assert not default_matmul()
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert default_matmul()

@@ -37,6 +37,7 @@ def default_matmul() -> bool:
     mm = torch.backends.cuda.matmul
     return (mm.allow_fp16_reduced_precision_reduction is True and mm.allow_bf16_reduced_precision_reduction is True
             and not mm.allow_fp16_accumulation and not torch.cuda.tunable.is_enabled()
+            and not torch.are_deterministic_algorithms_enabled()      # (torch.mm then refuses some settings)
             and torch.backends.cuda.preferred_blas_library() == torch._C._BlasBackend.Cublas)
 
 
