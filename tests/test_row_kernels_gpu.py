@@ -56,7 +56,8 @@ def test_swiglu_of_every_value(dtype):
     (768, 8, 1, 64, 640, 16, 128, 12, True), (1001, 8, 1, 64, 640, 0, 128, 0, False), (770, 4, 2, 64, 64, 16, 16, 4, True),
     (800, 3, 1, 128, 1040, 32, 0, 5, False), (900, 6, 2, 32, 192, 8, 24, 12, True),
     (800, 3, 1, 128, 1000, 64, 0, 128, False), (777, 5, 1, 16, 96, 8, 18, 3, True), (780, 11, 3, 64, 1024, 32, 100, 37, True),
-    (769, 9, 1, 128, 520, 32, 127, 0, True), (768, 1, 1, 32, 8, 16, 8, 1, False)])
+    (769, 9, 1, 128, 520, 32, 127, 0, True), (768, 1, 1, 32, 8, 16, 8, 1, False),
+    (768, 192, 12, 16, 64, 8, 16, 4, True)])     # (more gate weights than shared memory takes)
 def test_qkv_post_of_many_rows(dtype, n, H, K, hd, d, pairs, gate, ve, ring):
     from ultraviolet_b200 import _lib
     from ultraviolet_b200.kernels._util import DTYPE_CODE, stream_ptr

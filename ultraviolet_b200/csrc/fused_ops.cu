@@ -708,8 +708,8 @@ static int launch_qkv_post(const QkvPostParams& P, int hd, cudaStream_t st) {
                        (!P.ve_gate || aligned16(P.value_embed)) &&
                        (!P.k_cache || (((uintptr_t)P.k_cache | (uintptr_t)P.v_cache) & 7) == 0) &&
                        (!P.inv_freq || (P.rope_cs && (P.n_pairs == 8 || P.n_pairs == 16 || P.n_pairs == 32 || P.n_pairs == 64)));
-  if (rows_ok) {
-    const size_t smem = (size_t)((P.gate_out ? P.H : 0) + (P.ve_gate ? P.K : 0)) * QPR_GCH * sizeof(T);
+  const size_t smem = (size_t)((P.gate_out ? P.H : 0) + (P.ve_gate ? P.K : 0)) * QPR_GCH * sizeof(T);   // the gates' weights
+  if (rows_ok && smem <= 48 * 1024) {
     const int64_t ctas = ((int64_t)P.B + QPR_WARPS - 1) / QPR_WARPS;
     const unsigned grid = (unsigned)(ctas < 148 * 6 ? ctas : 148 * 6);
 #define UV_QKV_POST_ROWS(HD_)                                                                                             \

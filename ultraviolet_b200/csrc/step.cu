@@ -3,8 +3,8 @@
 // What bounds a step: with a few rows every kernel of a layer is a 3-5 us chain of dependent round trips on a mostly idle
 // GPU, and 70 of them in a row took 255-310 us at 1-48 rows, against 17 us of weight traffic.  Here a layer is six hops
 // between CTAs of 0.6-1.2 us each with 0.3-0.5 us of work in between (the attention: 2.3 us), and from some 16 rows on the
-// loads of CTAs that all read all rows (from L2, at a sixth of its rate): 100 us at 1 row, 110 at 8, 143 at 16, 175 at 32, 209 at 48 (UV-50M, contexts of
-// 200-900).
+// loads of CTAs that all read all rows (from L2, at a sixth of its rate): 100 us at 1 row, 110 at 8, 143 at 16, 175 at 32, 209
+// at 48 (UV-50M, contexts of 200-900).
 //
 // Split: one CTA per multiprocessor.  In the projections a CTA owns one 8-wide tile of output features (of gate | up up to
 // two pairs of tiles; UV-50M has 80, 80, 208 pairs and 80) for all rows, its weights in shared memory, fetched a layer
