@@ -101,3 +101,25 @@ def test_qkv_post_of_many_rows(dtype, n, H, K, hd, d, pairs, gate, ve, ring):
     assert int(o1) == int(o2) == (0 if ring else 2 * K)
     for a, b in zip((q1, g1, *c1), (q2, g2, *c2)):
         assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2])
+def test_qkv_post_takes_its_table_at_any_float(offset):
+    from ultraviolet_b200 import _lib
+    from ultraviolet_b200.kernels._util import stream_ptr
+    n, H, K, hd, d, pairs = 770, 2, 1, 64, 64, 16
+    g = torch.Generator(device="cuda").manual_seed(0)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    x, qkv0, pos = rnd(n, d).bfloat16(), rnd(n, (H + 2 * K) * hd).bfloat16(), torch.arange(n, device="cuda")
+    inv, table = rnd(pairs), rnd(n * 2 * pairs + offset)[offset:].view(n, 2 * pairs)
+    res = []
+    for cut in (n, 250):
+        qkv = qkv0.clone()
+        for a, b in _pieces(n, cut):
+            q = _lib.QkvArgs()
+            q.qkv, q.xn, q.pos = (t[a:b].data_ptr() for t in (qkv, x, pos))
+            q.inv_freq, q.rope_cs, q.dtype, q.xn_raw = inv.data_ptr(), table[a:b].data_ptr(), 2, 1
+            q.B, q.H, q.K, q.hd, q.d, q.n_pairs = b - a, H, K, hd, d, pairs
+            _lib.check(_lib.lib().uv_qkv_post_args(C.byref(q), stream_ptr(x.device)), "uv_qkv_post")
+        res.append(qkv)
+    assert torch.equal(*res) and not torch.equal(res[0], qkv0)

@@ -707,7 +707,8 @@ static int launch_qkv_post(const QkvPostParams& P, int hd, cudaStream_t st) {
                        (!P.ve_gate || P.ve_ch <= QPR_GCH) && aligned16(P.qkv) &&
                        (!P.ve_gate || aligned16(P.value_embed)) &&
                        (!P.k_cache || (((uintptr_t)P.k_cache | (uintptr_t)P.v_cache) & 7) == 0) &&
-                       (!P.inv_freq || (P.rope_cs && (P.n_pairs == 8 || P.n_pairs == 16 || P.n_pairs == 32 || P.n_pairs == 64)));
+                       (!P.inv_freq || (P.rope_cs && ((uintptr_t)P.rope_cs & 7) == 0 &&
+                                        (P.n_pairs == 8 || P.n_pairs == 16 || P.n_pairs == 32 || P.n_pairs == 64)));
   const size_t smem = (size_t)((P.gate_out ? P.H : 0) + (P.ve_gate ? P.K : 0)) * QPR_GCH * sizeof(T);   // the gates' weights
   if (rows_ok && smem <= 48 * 1024) {
     const int64_t ctas = ((int64_t)P.B + QPR_WARPS - 1) / QPR_WARPS;
