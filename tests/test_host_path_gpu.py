@@ -209,6 +209,8 @@ def test_watched_attention_calls_go_through_the_op():
             return super().__torch_function__(func, types, args, kwargs or {})
     f(b[0].as_subclass(Watch), *b[1:])
     assert any("decode_attn" in n for n in seen)
+    # a view that stands for other values than those in memory
+    assert torch.equal(f(torch._neg_view(b[0]), *b[1:]), f(-b[0], *b[1:]))
 
 
 def test_logits_keep_gradients_and_transforms():

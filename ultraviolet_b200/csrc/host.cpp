@@ -85,12 +85,14 @@ int code_of(at::ScalarType t) {
   }
 }
 
-// a tensor whose metadata and memory can be taken at face value on CUDA device `dev`
+// a tensor whose metadata and memory can be taken at face value on CUDA device `dev` (no wrapper, nor a view that stands for
+// other values than those in memory)
 bool plain(const Tensor& t, c10::Device dev) {
-  const c10::DispatchKeySet keys = t.unsafeGetTensorImpl()->key_set();
-  return t.defined() && t.device() == dev && t.layout() == at::kStrided && !keys.has(c10::DispatchKey::Python) &&
-         !keys.has(c10::DispatchKey::Functionalize) && !(t.requires_grad() && at::GradMode::is_enabled()) &&
-         !t._fw_grad(0).defined();
+  constexpr c10::DispatchKeySet others({c10::DispatchKey::Python, c10::DispatchKey::Functionalize, c10::DispatchKey::Negative,
+                                        c10::DispatchKey::Conjugate, c10::DispatchKey::ZeroTensor,
+                                        c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper});
+  return t.defined() && t.device() == dev && t.layout() == at::kStrided && !t.key_set().has_any(others) &&
+         !(t.requires_grad() && at::GradMode::is_enabled()) && !t._fw_grad(0).defined();
 }
 // nothing watches or rewrites the calls of this thread: no dispatch or function mode, transform or tracer
 bool modes_off() {
